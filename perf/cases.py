@@ -1,7 +1,7 @@
 """What the performance of this repository is measured on: the linear layers of decoder models whose
 weights are GGUF blocks, driven through `brotensor_b200.ops` as an inference program drives them.
 
-A case is one of five kinds of pass:
+A case is one of four kinds of pass:
 
   step    one decode step of `layers` layers for `rows` sequences and, with `vocab`, the LM head. A decode
           loop captures its step once and replays it per token, so `prepare` captures and `run` replays.
