@@ -147,21 +147,31 @@ def _biases(d, case, dtype):
     return {n: d.normal(1, rows, dtype).view(-1) if case["bias"] and n in "qkv" else None for n, _, rows, _ in _layer(case)}
 
 
+def _step_inputs(case, d):
+    """Raw GGUF weights and biases of each layer, the head and the activations, in the order they are drawn."""
+    dt, m, h, f = _DT[case["dtype"]], case["rows"], case["hidden"], case["ffn"]
+    layers = []
+    for _ in range(case["layers"]):
+        W = {n: d.weight(fmt, rows, k) for n, fmt, rows, k in _layer(case)}
+        layers.append((W, _biases(d, case, dt)))
+    head = d.weight(_MIX[case["mix"]][1], case["vocab"], h)
+    x, a, hf = d.normal(m, h, dt), d.normal(m, h, dt), d.gated(m, f, dt)
+    gamma = (torch.rand(h, device="cuda", generator=d.g) + 0.5).to(dt)
+    return layers, head, x, a, hf, gamma
+
+
 def _prepare_step(case, d):
     dt, m = _DT[case["dtype"]], case["rows"]
     h, f, L = case["hidden"], case["ffn"], case["layers"]
     head_fmt = _MIX[case["mix"]][1]
     specs = _layer(case)
+    raw, head, x, a, hf, gamma = _step_inputs(case, d)
     layers = []
-    for _ in range(L):
-        W = {n: d.weight(fmt, rows, k) for n, fmt, rows, k in specs}
+    for W, B in raw:
         F = {n: fmt for n, fmt, _, _ in specs}
         if case["repack"]:  # a program that never reads the weights back regroups them once, at load
             W["down"], F["down"] = ops.repack(F["down"], W["down"], h, f), ops.repacked_fmt(F["down"], f)
-        layers.append((W, F, _biases(d, case, dt)))
-    head = d.weight(head_fmt, case["vocab"], h)
-    x, a, hf = d.normal(m, h, dt), d.normal(m, h, dt), d.gated(m, f, dt)
-    gamma = (torch.rand(h, device="cuda", generator=d.g) + 0.5).to(dt)
+        layers.append((W, F, B))
     yt = torch.float16 if dt == torch.float16 else torch.float32
     names = [("act", f) if n == "gate" else (n, rows) for n, _, rows, _ in specs if n != "up"] if case["fused"] else [(n, rows) for n, _, rows, _ in specs]
     Y = {n: torch.empty(L, m, rows, dtype=yt, device="cuda") for n, rows in names}
@@ -207,6 +217,12 @@ def _run_prompt(s):
     return out
 
 
+def _prepare_call(case, d):
+    fmt, dt = _MIX[case["fmt"]][0], _DT[case["dtype"]]
+    return dict(kind="call", fmt=fmt, n=case["n"], w=d.weight(fmt, case["n"], case["k"]), x=d.normal(case["rows"], case["k"], dt),
+                b=d.normal(1, case["n"], dt).view(-1) if case["bias"] else None)
+
+
 def prepare(case, seed):
     d = _Draw(seed)
     if case["kind"] == "step":
@@ -215,9 +231,7 @@ def prepare(case, seed):
         return dict(kind="prompt", **_prepare_prompt(case, d))
     if case["kind"] == "decode":
         return dict(kind="decode", dt=_DT[case["dtype"]], mats=[(fmt, d.weight(fmt, n, k), n, k) for _, fmt, n, k in _layer(case)])
-    fmt, dt = _MIX[case["fmt"]][0], _DT[case["dtype"]]
-    return dict(kind="call", fmt=fmt, n=case["n"], w=d.weight(fmt, case["n"], case["k"]), x=d.normal(case["rows"], case["k"], dt),
-                b=d.normal(1, case["n"], dt).view(-1) if case["bias"] else None)
+    return _prepare_call(case, d)
 
 
 def run(s):
@@ -229,6 +243,81 @@ def run(s):
     if s["kind"] == "decode":
         return [ops.dequant(fmt, w, n, k, s["dt"]) for fmt, w, n, k in s["mats"]]
     return ops.linear(s["fmt"], s["w"], s["x"], s["n"], bias=s["b"])
+
+
+# ---- the same passes in 64 bits ---------------------------------------------------------------------------
+
+def _f16(b):
+    return b.contiguous().view(torch.float16).double()
+
+
+def _k_scales(b):
+    """The eight 6-bit scales and mins in the 12 bytes of a Q4_K / Q5_K block."""
+    s0, s1, s2 = b[:, 4:8], b[:, 8:12], b[:, 12:16]
+    sc = torch.cat([s0 & 63, (s2 & 15) | (s0 >> 6) << 4], 1)
+    m = torch.cat([s1 & 63, (s2 >> 4) | (s1 >> 6) << 4], 1)
+    return sc.double(), m.double()
+
+
+def _rows64(fmt, raw, n, k):
+    """Blocks (the block formats of ggml) -> (n, k) in 64 bits."""
+    b = raw.view(-1, synth.BLOCK_BYTES[fmt])
+    if fmt == synth.Q8_0:
+        w = _f16(b[:, 0:2]) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif fmt == synth.Q4_0:
+        w = _f16(b[:, 0:2]) * (torch.cat([b[:, 2:] & 15, b[:, 2:] >> 4], 1).double() - 8)
+    elif fmt == synth.Q6_K:
+        ql, qh = b[:, :128].reshape(-1, 2, 2, 32), b[:, 128:192].reshape(-1, 2, 32)
+        q = torch.stack([(ql[:, :, j & 1] >> 4 * (j >> 1) & 15) | (qh >> 2 * j & 3) << 4 for j in range(4)], 2).double() - 32
+        sc = b[:, 192:208].contiguous().view(torch.int8).double()
+        w = q.reshape(-1, 16, 16) * (_f16(b[:, 208:210]) * sc).unsqueeze(2)
+    else:
+        sc, m = _k_scales(b)
+        qs = b[:, -128:].reshape(-1, 4, 1, 32)
+        q = torch.cat([qs & 15, qs >> 4], 2).reshape(-1, 8, 32)
+        if fmt == synth.Q5_K:
+            q = q | torch.stack([b[:, 16:48] >> j & 1 for j in range(8)], 1) << 4
+        w = (_f16(b[:, 0:2]) * sc).unsqueeze(2) * q.double() - (_f16(b[:, 2:4]) * m).unsqueeze(2)
+    return w.reshape(n, k)
+
+
+def _linear64(fmt, raw, x, n, bias=None):
+    k = x.shape[1]
+    y, step = [], max(1, (1 << 24) // k)
+    blocks = raw.view(n, -1)
+    for r in range(0, n, step):
+        part = blocks[r:r + step]
+        y.append(x.double() @ _rows64(fmt, part.reshape(-1), part.shape[0], k).T)
+    y = torch.cat(y, 1)
+    return y if bias is None else y + bias.double()
+
+
+def exact(case, seed):
+    d = _Draw(seed)
+    if case["kind"] == "decode":
+        return [_rows64(fmt, d.weight(fmt, n, k), n, k) for _, fmt, n, k in _layer(case)]
+    if case["kind"] == "call":
+        s = _prepare_call(case, d)
+        return _linear64(s["fmt"], s["w"], s["x"], s["n"], s["b"])
+    fmt = _MIX[case["mix"]][1]
+    if case["kind"] == "prompt":
+        s = _prepare_prompt(case, d)
+        rows = s["table"].view(case["vocab"], -1)[s["ids"].long()]
+        out = [_rows64(fmt, rows.reshape(-1), rows.shape[0], case["hidden"])]
+        for W, B in s["layers"]:
+            out += [_linear64(f, W[n], s["a"] if n == "o" else s["hf"] if n == "down" else s["x"], rows, B[n]) for n, f, rows, _ in _layer(case)]
+        return out + [_linear64(fmt, s["head"], s["x"][-1:], case["vocab"])]
+    layers, head, x, a, hf, gamma = _step_inputs(case, d)
+    x64 = x.double()
+    normed = x64 * torch.rsqrt(x64.square().mean(1, keepdim=True) + 1e-5) * gamma.double()
+    Y = {}
+    for W, B in layers:
+        for n, f, rows, _ in _layer(case):
+            src = a if n == "o" else hf if n == "down" else normed if case["fused"] and n in "qkv" else x
+            Y.setdefault(n, []).append(_linear64(f, W[n], src, rows, B[n]))
+    if case["fused"]:
+        Y["gate"] = [torch.nn.functional.silu(g) * u for g, u in zip(Y["gate"], Y.pop("up"))]
+    return [torch.stack(v) for v in Y.values()] + [_linear64(fmt, head, x, case["vocab"])]
 
 
 # ---- what a pass cannot do without -----------------------------------------------------------------------
