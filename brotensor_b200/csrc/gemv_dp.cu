@@ -104,8 +104,8 @@ __device__ __forceinline__ void stage_x16(const StreamParams& p, uint32_t sbase,
             for (int u = 0; u < 4; ++u) {
                 const int idx = min(base + u * nthreads, total - 1), m = idx / segs, seg = idx - m * segs;
                 const float4* X = reinterpret_cast<const float4*>(static_cast<const float*>(p.X) + (size_t)m * p.K) + 2 * seg;
-                r[u][0] = __ldg(X);
-                r[u][1] = __ldg(X + 1);
+                r[u][0] = ld_dep_f4(X);
+                r[u][1] = ld_dep_f4(X + 1);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -117,7 +117,7 @@ __device__ __forceinline__ void stage_x16(const StreamParams& p, uint32_t sbase,
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int idx = min(base + u * nthreads, total - 1), m = idx / segs, seg = idx - m * segs;
-                r[u] = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.X) + (size_t)m * p.K) + seg);
+                r[u] = ld_dep_u4(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.X) + (size_t)m * p.K) + seg);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -900,9 +900,21 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * NG * 32, 1) gemv_dp_ker
     TRACE_STAMP(tid == 0, 1);
 
     if (warp >= kConsumers) {
-        // ---- producer of pipeline g: weights do not depend on the stream-ordered
-        // predecessor, so the copies start before griddepcontrol.wait
+        // ---- producer of pipeline g. The predecessor may be what writes the weights (an upload, a repack):
+        // unless the caller has said otherwise (early_w) they are read after griddepcontrol.wait.
         const int g = warp - kConsumers;
+        if (!p.early_w) {
+            if (g < n_tiles) {  // the first stage's rows: into the L2 meanwhile
+                const TileRef tr = tile_ref<EXT>(p, row_begin + g * TR);
+                const int nrows = min(min(TR, row_end - (row_begin + g * TR)), tr.N - tr.row0);
+                if (lane < nrows) {
+                    const uint8_t* src = ((EXT & kExtSwiglu) && p.W_up) ? (((lane & 1) ? p.W_up : tr.W) + (size_t)((tr.row0 + lane) >> 1) * p.row_bytes)
+                                                                        : (tr.W + (size_t)(tr.row0 + lane) * p.row_bytes);
+                    bulk_prefetch_l2(src, (uint32_t)min(p.slice_chunks, p.chunks_per_row) * Chunk<FMT>::bytes);
+                }
+            }
+            grid_dep_wait();
+        }
         const uint32_t ring = sbase + (uint32_t)(p.off_stage + g * p.n_stages * stage_bytes);
         int slot = 0;
         uint32_t phase = 0;
@@ -1291,17 +1303,9 @@ static int launch_dp_k(const StreamParams& p_in, int grid, size_t smem, cudaStre
         B200Q_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((kConsumerWarps + 1) * NG * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = stream_get_option(1) ? 1 : 0;
-    B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+    // (two to four rows: plain launches, under which reading the weights at once is no question)
+    p.early_w = MT > 1 || pdl_option() != 0;
+    B200Q_CUDA_TRY(launch_dep(MT == 1 ? pdl_option() >= 0 : pdl_option() > 0, kern, dim3((unsigned)grid), dim3((kConsumerWarps + 1) * NG * 32), smem, st, p));
     return B200Q_OK;
 }
 

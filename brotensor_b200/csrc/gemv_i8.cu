@@ -366,7 +366,7 @@ static int launch_i8(const I8Params& p, int grid, size_t smem, cudaStream_t st) 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = stream_get_option(1) ? 1 : 0;
+    cfg.numAttrs = stream_get_option(1) > 0 ? 1 : 0;
     B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
     return B200Q_OK;
 }

@@ -601,7 +601,7 @@ static int launch_stream_k(const StreamPlan& pl, cudaStream_t st) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_opt_pdl ? 1 : 0;
+    cfg.numAttrs = g_opt_pdl > 0 ? 1 : 0;
     B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, pl.p));
     return B200Q_OK;
 }

@@ -61,6 +61,7 @@ struct XrParams {
     int n_slots;         // ring depth in row pairs
     int pair_q, pair_r;  // CTA b owns pair_q + (b < pair_r) row pairs, starting at b * pair_q + min(b, pair_r)
     unsigned int wait_limit_us;
+    int early_w;         // 1: weights are read ahead of griddepcontrol.wait
 #ifdef B200Q_TRACE
     unsigned long long* trace;
 #endif
@@ -230,8 +231,8 @@ __global__ void __launch_bounds__(CW * 32, 1) gemv_xr_kernel(const __grid_consta
     // (n_slots is a multiple of CW), and its first lane issues the copy of the item that will use a slot
     // next as soon as the warp is done with the slot. No producer warp, no "empty" barriers, and a slot
     // meets one warp only, in order, so a barrier's two parities cannot be mistaken for one another.
-    // Weights do not depend on the stream-ordered predecessor: the first copies go out before
-    // griddepcontrol.wait.
+    // The predecessor may be what writes the weights: unless the caller has said otherwise (early_w) the first
+    // copies go out right after griddepcontrol.wait, their bytes on the way to the L2 meanwhile.
     if (tid == 0) abort_flag = 0;
     // The copy of item `it` into its slot; called by a warp's first lane.
     auto feed = [&](int it, int s) {
@@ -249,7 +250,11 @@ __global__ void __launch_bounds__(CW * 32, 1) gemv_xr_kernel(const __grid_consta
     if (lane == 0) {
         for (int s = warp; s < p.n_slots; s += CW) mbar_init(smem_u32(&bar_full[s]), 1);
         fence_mbar_init();
-        feed(warp, warp);
+        if (p.early_w) feed(warp, warp);
+        else if (warp < n_items) {
+            const int row = 2 * (pair_first + warp);
+            bulk_prefetch_l2(p.W + (size_t)row * p.row_bytes, (uint32_t)min(2, p.N - row) * (uint32_t)p.row_bytes);
+        }
     }
     TRACE_STAMP(tid == 0, 7);
     grid_dep_launch();
@@ -257,6 +262,7 @@ __global__ void __launch_bounds__(CW * 32, 1) gemv_xr_kernel(const __grid_consta
 
     // ---- consumers
     grid_dep_wait();  // activations (and Y) belong to the stream-ordered predecessor
+    if (lane == 0 && !p.early_w) feed(warp, warp);
     TRACE_STAMP(tid == 0, 2);
     {
         // K % 256 == 0 and CW * 32 % 32 == 0: whole warps are in or out. All of a thread's loads go out
@@ -271,8 +277,8 @@ __global__ void __launch_bounds__(CW * 32, 1) gemv_xr_kernel(const __grid_consta
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const float4* X = reinterpret_cast<const float4*>(p.X) + 2 * min(tid + u * CW * 32, segs - 1);
-                r[u][0] = __ldg(X);
-                r[u][1] = __ldg(X + 1);
+                r[u][0] = ld_dep_f4(X);
+                r[u][1] = ld_dep_f4(X + 1);
             }
             if (lane == 0) feed(warp + CW, warp + CW);
 #pragma unroll
@@ -283,7 +289,7 @@ __global__ void __launch_bounds__(CW * 32, 1) gemv_xr_kernel(const __grid_consta
         } else {
             uint4 r[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) r[u] = __ldg(reinterpret_cast<const uint4*>(p.X) + min(tid + u * CW * 32, segs - 1));
+            for (int u = 0; u < U; ++u) r[u] = ld_dep_u4(reinterpret_cast<const uint4*>(p.X) + min(tid + u * CW * 32, segs - 1));
             if (lane == 0) feed(warp + CW, warp + CW);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -492,6 +498,7 @@ static int launch_gemv_xr_cw(int fmt, const void* W, const void* X, int x_dtype,
     if (slots < CW) return B200Q_OK;
     p.n_slots = slots;
     p.wait_limit_us = (unsigned int)dp_get_wait_limit_us();
+    p.early_w = pdl_option() != 0;
 #ifdef B200Q_TRACE
     p.trace = dp_trace_next(grid);
 #endif
@@ -507,17 +514,7 @@ static int launch_gemv_xr_cw(int fmt, const void* W, const void* X, int x_dtype,
         B200Q_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(CW * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = stream_get_option(1) ? 1 : 0;
-    B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+    B200Q_CUDA_TRY(launch_dep(pdl_option() >= 0, kern, dim3((unsigned)grid), dim3(CW * 32), smem, st, p));
     *taken = true;
     return B200Q_OK;
 }

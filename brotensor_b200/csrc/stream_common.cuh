@@ -34,6 +34,7 @@ struct StreamParams {
     // split_q + (b < split_r) of them, starting at b * split_q + min(b, split_r) (no division on the device).
     int split_q, split_r;
     unsigned int wait_limit_us;  // bound of the device-side waits in microseconds (0: one second)
+    int early_w;                 // 1: weights are read ahead of griddepcontrol.wait
     int step_fill;               // 1: only the first stage of a pipeline is requested ahead of the activation loads
 #ifdef B200Q_TRACE
     unsigned long long* trace;  // trace builds: sixteen %globaltimer stamps per CTA of this launch
