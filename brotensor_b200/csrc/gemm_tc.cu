@@ -197,8 +197,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
 
 static int round_up16(int v) { return (v + 15) & ~15; }
 
-int launch_gemm_pair_pass(int fmt, const void* W, const uint8_t* Xp, int tok_stride, const void* bias, int bias_dtype,
-                          void* Y, int y_dtype, int tokens, int N, int K, int n_split, float* ypart, int* status, cudaStream_t st);
+int launch_gemm_pair(int fmt, const void* W, const uint8_t* Xp, int tok_stride, const void* bias, int bias_dtype, void* Y, int y_dtype,
+                     int tokens, int tok_pass, int N, int K, int n_split, float* ypart, int* status, cudaStream_t st);
 // non-zero: passes run on CTA pairs (gemm_tc2.cu, the default); 0: one CTA per 128 weight rows
 // (this file; kept as the reference the pair kernel is compared with bit for bit)
 static int g_gemm_pair = -1;
@@ -213,21 +213,41 @@ static bool gemm_tc_takes(int fmt, const void* W, int M, int K) {
     return fmt == kQ4_K || fmt == kQ6_K || fmt == kQ8_0;
 }
 
-// Split K. A pass runs one CTA pair per 256 weight rows: 4096 rows are 16 pairs on 32 of the 148 SMs.
-// With at most half of the SMs busy the k-blocks of a row tile are split over up to eight pairs
-// (equal shares, whole 256-element blocks, at least eight k-blocks each); the partial sums go through
-// the workspace and are added in a fixed order. 1 = no split.
+// How a call is cut into work for the 74 CTA pairs of the chip: passes of up to 512 tokens (each decodes the weights
+// again), and K splits (equal shares, whole 256-element blocks, at least eight k-blocks each; the partial sums go through the
+// workspace and are added in a fixed order by a second kernel). One launch holds all of it, so the plan is the one whose waves
+// take least by this model (us, fitted to B200): a 64-k stage costs the larger of its MMAs (0.85 for 512 tokens) and its
+// decode; a tile adds its start and epilogue; split sums are written and read once. Passes launched one after the other
+// left most pairs idle - 2000 tokens of 4096 rows were four launches of 16 tiles, split in four - and 400 tokens a pass
+// beat 512 where 56 row tiles make 280 = 3.8 instead of 224 = 3.03 waves.
 static int g_gemm_split = 1;
 void gemm_set_split(int v) { g_gemm_split = v ? 1 : 0; }
 int gemm_get_split() { return g_gemm_split; }
-static int gemm_split_factor(int fmt, int N, int K) {
-    if (!g_gemm_split || g_gemm_pair == 0 || N % 4 != 0) return 1;
-    const int pairs = ((N + kGemmRows - 1) / kGemmRows + 1) / 2, n_kb = K / kBK;
-    if (pairs > 37) return 1;
-    int s = 74 / pairs;
-    if (s > 8) s = 8;
-    while (s > 1 && (n_kb % (4 * s) != 0 || n_kb / s < 8)) --s;
-    return s;
+struct GemmPlan {
+    int tok_pass, split;
+};
+static GemmPlan gemm_plan(int fmt, int M, int N, int K, bool may_split) {
+    const int pairs = ((N + kGemmRows - 1) / kGemmRows + 1) / 2, n_kb = K / kBK, chip = 74;
+    const double decode = (fmt == kQ6_K || fmt == kQ6_KP) ? 1.05 : fmt == kQ8_0 ? 0.75 : 0.69;
+    const int p_min = (M + kMaxTokens - 1) / kMaxTokens;
+    GemmPlan best = {kMaxTokens, 1};
+    double best_t = -1;
+    for (int p = p_min; p <= 2 * p_min + 2; ++p) {
+        const int pass = p == 1 ? round_up16(M) : ((M + p - 1) / p + 31) & ~31, passes = (M + pass - 1) / pass;
+        if (p > p_min && pass < 128) break;
+        for (int s = 1; s <= 8; ++s) {
+            if (s > 1 && (!may_split || !g_gemm_split || N % 4 != 0 || n_kb % (4 * s) != 0 || n_kb / s < 8)) continue;
+            const int waves = (pairs * passes * s + chip - 1) / chip;
+            const double stage = 0.85 * pass / 512 > decode ? 0.85 * pass / 512 : decode;
+            double t = waves * ((double)n_kb / s * stage + 3.0 + 4.0 * pass / 512);
+            if (s > 1) t += 2.5 + (double)s * M * N * 8 / 5.0e6;
+            if (best_t < 0 || t < best_t * 0.98) {  // fewer passes and splits on a tie
+                best_t = t;
+                best = {pass, s};
+            }
+        }
+    }
+    return best;
 }
 static size_t gemm_xp_bytes(int M, int K) { return ((size_t)(K / kBK) * (size_t)round_up16(M) * 128u + 255u) & ~(size_t)255u; }
 
@@ -241,8 +261,9 @@ size_t gemm_tc_workspace_min_bytes(int fmt, int x_dtype, int M, int N, int K) {
 size_t gemm_tc_workspace_bytes(int fmt, int x_dtype, int M, int N, int K) {
     (void)x_dtype;
     if (!gemm_tc_takes(fmt, nullptr, M, K)) return 0;
-    const int s = gemm_split_factor(fmt, N, K);
-    return gemm_xp_bytes(M, K) + (s > 1 ? (size_t)s * (size_t)(M < kMaxTokens ? M : kMaxTokens) * N * sizeof(float) : 0);
+    const int s = gemm_plan(fmt, M, N, K, g_gemm_pair != 0).split;
+    const size_t rows = M <= kMaxTokens ? M : (size_t)((M + kMaxTokens - 1) / kMaxTokens) * kMaxTokens;
+    return gemm_xp_bytes(M, K) + (s > 1 ? s * rows * N * sizeof(float) : 0);
 }
 
 template <int FMT>
@@ -270,7 +291,7 @@ int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const voi
     // (the reduction kernel moves four neighbouring outputs at a time: Y and an FP32 bias must be aligned for that)
     const bool quads_ok = (reinterpret_cast<uintptr_t>(Y) & (y_dtype == B200Q_DT_F32 ? 15 : 3)) == 0 &&
                           (!bias || x_dtype != B200Q_DT_F32 || (reinterpret_cast<uintptr_t>(bias) & 15) == 0);
-    const int n_split = ws && quads_ok && ws_bytes >= gemm_tc_workspace_bytes(fmt, x_dtype, M, N, K) ? gemm_split_factor(fmt, N, K) : 1;
+    const GemmPlan plan = gemm_plan(fmt, M, N, K, g_gemm_pair != 0 && ws && quads_ok && ws_bytes >= gemm_tc_workspace_bytes(fmt, x_dtype, M, N, K));
     if (!ws || ws_bytes < need) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
     if (reinterpret_cast<uintptr_t>(ws) & 255) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace must be 256-byte aligned");
     const int tok_total = round_up16(M);
@@ -285,15 +306,10 @@ int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const voi
         B200Q_CUDA_TRY(cudaGetLastError());
     }
     const int ysz = y_dtype == B200Q_DT_F32 ? 4 : 2;
+    if (g_gemm_pair != 0)
+        return launch_gemm_pair(fmt, W, static_cast<const uint8_t*>(ws), tok_total, bias, x_dtype, Y, y_dtype, M, plan.tok_pass, N, K, plan.split,
+                                reinterpret_cast<float*>(static_cast<char*>(ws) + gemm_xp_bytes(M, K)), status, st);
     for (int t0 = 0; t0 < M; t0 += kMaxTokens) {
-        if (g_gemm_pair != 0) {
-            const int tokens = M - t0 < kMaxTokens ? M - t0 : kMaxTokens;
-            if (int rc = launch_gemm_pair_pass(fmt, W, static_cast<const uint8_t*>(ws) + (size_t)t0 * 128u, tok_total, bias, x_dtype,
-                                               static_cast<char*>(Y) + (size_t)t0 * N * ysz, y_dtype, tokens, N, K, n_split,
-                                               reinterpret_cast<float*>(static_cast<char*>(ws) + gemm_xp_bytes(M, K)), status, st))
-                return rc;
-            continue;
-        }
         GemmParams p = {};
         p.W = static_cast<const uint8_t*>(W);
         p.Xp = static_cast<const uint8_t*>(ws) + (size_t)t0 * 128u;

@@ -35,15 +35,16 @@ constexpr int kPairMaxStages = 8;
 
 struct PairParams {
     const uint8_t* W;
-    const uint8_t* Xp;   // prepared activations of this pass: [K/64][tok_stride][64] FP16, swizzled rows
+    const uint8_t* Xp;   // prepared activations: [K/64][tok_stride][64] FP16, swizzled rows
     const void* bias;
     void* Y;
     int* status;
-    int tokens, tok_pad, xp_tok_stride;
+    int tokens, xp_tok_stride;
+    int tok_pass;        // blockIdx.z = z works on tokens [z * tok_pass, + tok_pass), at most 512 (a multiple of 16)
     int N, K, row_bytes;
     int bias_dtype, y_dtype;
     int n_a, n_b;        // ring depths in k-blocks: decoded weights (16 KB slots) and slabs; n_b <= n_a
-    int g_bytes;         // bytes of one token group's half in a slab slot: (min(tok_pad, 256) / 2) * 128
+    int g_bytes;         // bytes of one token group's half in a slab slot: (min(tok_pass, 256) / 2) * 128
     int b_bytes;         // one slab slot of this CTA: g_bytes * groups
     // Split K (few row tiles, long rows): blockIdx.y = s works on k-blocks [s * kb_split, (s + 1) * kb_split) and
     // writes its FP32 partial sums, without bias, to Ypart[s][token][N]; a second kernel adds them up in order.
@@ -205,10 +206,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
     const uint32_t crank = cluster_ctarank();         // 0 = leader
     const int row0 = blockIdx.x * kGemmRows;          // the pair's CTAs own consecutive row tiles
     const int n_kb = p.n_split > 1 ? p.kb_split : p.K / kBK;  // k-blocks of this CTA; its first one is blockIdx.y * kb_split
-    const uint32_t tmem_cols = p.tok_pad <= 32 ? 32u : p.tok_pad <= 64 ? 64u : p.tok_pad <= 128 ? 128u : p.tok_pad <= 256 ? 256u : 512u;
+    const int t0 = (int)blockIdx.z * p.tok_pass, tokens = min(p.tok_pass, p.tokens - t0), tok_pad = (tokens + 15) & ~15;
+    const uint8_t* const xp = p.Xp + (size_t)t0 * 128u;
+    const uint32_t tmem_cols = tok_pad <= 32 ? 32u : tok_pad <= 64 ? 64u : tok_pad <= 128 ? 128u : tok_pad <= 256 ? 256u : 512u;
     // token groups of up to 256: group g is one MMA of N = ng tokens into accumulator columns 256 g ..;
     // this CTA holds tokens [256 g + crank * ng / 2, + ng / 2) of it
-    const int n0 = min(p.tok_pad, 256), n1 = p.tok_pad - n0;
+    const int n0 = min(tok_pad, 256), n1 = tok_pad - n0;
     const int groups = n1 > 0 ? 2 : 1;
 
     if (tid == 0) {
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
                 const uint32_t full = smem_u32(&bar_b_full[bs]);
                 const uint32_t h0 = (uint32_t)(n0 / 2) * 128u, h1 = (uint32_t)(n1 / 2) * 128u;
                 mbar_arrive_expect_tx(full, h0 + h1);
-                const uint8_t* src = p.Xp + (size_t)(kb + (int)blockIdx.y * p.kb_split) * p.xp_tok_stride * 128u;
+                const uint8_t* src = xp + (size_t)(kb + (int)blockIdx.y * p.kb_split) * p.xp_tok_stride * 128u;
                 const uint32_t dst = b_base + bs * p.b_bytes;
                 bulk_g2s(dst, src + (size_t)crank * h0, h0, full);
                 if (groups == 2) bulk_g2s(dst + p.g_bytes, src + 256u * 128u + (size_t)crank * h1, h1, full);
@@ -485,24 +488,24 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
                 else bv = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
             }
             const uint32_t tlane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            const int share = ((p.tok_pad / 16 + 1) / 2) * 16;
-            const int cbeg = H * share, cend = min(cbeg + share, p.tok_pad);
+            const int share = ((tok_pad / 16 + 1) / 2) * 16;
+            const int cbeg = H * share, cend = min(cbeg + share, tok_pad);
             for (int c0 = cbeg; c0 < cend; c0 += 16) {
                 uint32_t r[16];
                 tmem_ld16(tlane + (uint32_t)c0, r);
                 tmem_ld_wait();
                 if (n < p.N && p.n_split > 1) {
-                    float* part = p.Ypart + (size_t)blockIdx.y * p.tokens * p.N;
+                    float* part = p.Ypart + ((size_t)blockIdx.y * p.tokens + t0) * p.N;
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (c0 + j < p.tokens) part[(size_t)(c0 + j) * p.N + n] = __uint_as_float(r[j]);
+                        if (c0 + j < tokens) part[(size_t)(c0 + j) * p.N + n] = __uint_as_float(r[j]);
                 } else if (n < p.N) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int t = c0 + j;
-                        if (t < p.tokens) {
+                        if (t < tokens) {
                             const float v = __uint_as_float(r[j]) + bv;
-                            const size_t o = (size_t)t * p.N + n;
+                            const size_t o = (size_t)(t0 + t) * p.N + n;
                             if (p.y_dtype == B200Q_DT_F32) static_cast<float*>(p.Y)[o] = v;
                             else if (p.y_dtype == B200Q_DT_F16) static_cast<__half*>(p.Y)[o] = __float2half_rn(v);
                             else static_cast<__nv_bfloat16*>(p.Y)[o] = __float2bfloat16_rn(v);
@@ -537,7 +540,7 @@ static int launch_pair_fmt(const PairParams& p, size_t smem, cudaStream_t st) {
     }
     const unsigned tiles = (unsigned)((p.N + kGemmRows - 1) / kGemmRows);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((tiles + 1u) & ~1u, (unsigned)(p.n_split > 1 ? p.n_split : 1));  // whole pairs; a CTA past the last row tile decodes row N-1 and stores nothing
+    cfg.gridDim = dim3((tiles + 1u) & ~1u, (unsigned)(p.n_split > 1 ? p.n_split : 1), (unsigned)((p.tokens + p.tok_pass - 1) / p.tok_pass));  // whole pairs; a CTA past the last row tile decodes row N-1 and stores nothing
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -590,11 +593,10 @@ __global__ void __launch_bounds__(256) gemm_split_reduce_kernel(const float* __r
     }
 }
 
-// One pass (<= 512 tokens) of the prefill GEMM on CTA pairs. The caller has run the activation
-// pre-pass; Xp points at this pass's first token row inside the workspace. n_split > 1: K is split
-// over blockIdx.y and `ypart` (n_split * tokens * N floats) takes the partial sums.
-int launch_gemm_pair_pass(int fmt, const void* W, const uint8_t* Xp, int tok_stride, const void* bias, int bias_dtype,
-                          void* Y, int y_dtype, int tokens, int N, int K, int n_split, float* ypart, int* status, cudaStream_t st) {
+// The prefill GEMM on CTA pairs, all tokens in one launch of passes of `tok_pass` (at most 512). The caller has run the
+// activation pre-pass. n_split > 1: K is split over blockIdx.y and `ypart` (n_split * tokens * N floats) takes the partial sums.
+int launch_gemm_pair(int fmt, const void* W, const uint8_t* Xp, int tok_stride, const void* bias, int bias_dtype, void* Y, int y_dtype,
+                     int tokens, int tok_pass, int N, int K, int n_split, float* ypart, int* status, cudaStream_t st) {
     PairParams p = {};
     p.n_split = n_split > 1 ? n_split : 1;
     p.kb_split = (K / kBK) / p.n_split;
@@ -608,15 +610,15 @@ int launch_gemm_pair_pass(int fmt, const void* W, const uint8_t* Xp, int tok_str
     p.Y = Y;
     p.status = status;
     p.tokens = tokens;
-    p.tok_pad = (tokens + 15) & ~15;
+    p.tok_pass = tok_pass;
     p.xp_tok_stride = tok_stride;
     p.N = N;
     p.K = K;
     p.row_bytes = (K / b200q_block_elems(fmt)) * b200q_block_bytes(fmt);
     p.bias_dtype = bias_dtype;
     p.y_dtype = y_dtype;
-    const int n0 = p.tok_pad < 256 ? p.tok_pad : 256;
-    const int groups = p.tok_pad > 256 ? 2 : 1;
+    const int n0 = tok_pass < 256 ? tok_pass : 256;
+    const int groups = tok_pass > 256 ? 2 : 1;
     p.g_bytes = (n0 / 2) * 128;
     p.b_bytes = p.g_bytes * groups;
     // Ring depths: slabs three k-blocks ahead (they come from L2 with about a microsecond of latency), decoded

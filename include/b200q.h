@@ -212,7 +212,8 @@ int b200q_gemv_shard_topk(int fmt, const void* W_shard, const void* x, int x_dty
  * `ws` is caller-owned scratch of at least b200q_gemm_workspace_bytes() bytes,
  * 256-byte aligned (it holds the activations converted to the operand layout
  * and, for matrices of few rows, whose k range is split over several CTA
- * pairs, the FP32 partial sums: splits x min(M, 512) x N floats);
+ * pairs, the FP32 partial sums: splits x M x N floats, M above 512
+ * rounded up to a multiple of it);
  * it may be NULL when that size is 0. Calls that share a workspace must be
  * ordered on one stream.
  * Replaces the tensor-core branch of linear_forward_batched_q4k_fp16 / _q6k_ /
@@ -285,7 +286,7 @@ int b200q_device_status(int* status_out);
  *                 of Q6_K from 8192 weight rows, which run as two passes of the small-batch GEMV), 1 = passes of the
  *                 decode GEMV only, 2 = the tcgen05 GEMM or an error
  *   "gemm_pair"   0 = one-CTA tcgen05 kernel, otherwise the CTA-pair kernel (default)
- *   "gemm_split"  0 = never split K; 1 (default) = matrices whose row tiles occupy at most half of the SMs
+ *   "gemm_split"  0 = never split K; 1 (default) = where it shortens the call, matrices of few row tiles
  *                 (N <= 9472) have their k-blocks split over up to eight CTA pairs, partial sums added in a
  *                 fixed order by a second kernel (b200q_gemm_workspace_bytes() grows accordingly)
  *   "gemv_xr"     Q4_K / Q6_K, one activation row, K <= 4096: 1 = the activation-resident kernel where it is the

@@ -1,0 +1,35 @@
+"""How a long prompt is cut into token passes and K splits inside one launch of the prefill GEMM: token counts around the
+passes' edges (one token into a second pass, a last pass of a few tokens, several passes with and without a split K) against the
+oracle on a sample of the columns (prefill bound, rel-L2 <= 2e-3), and against the one-CTA kernel, which takes 512 tokens after another."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle
+from brotensor_b200 import synth
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,N,K,M", [(synth.Q4_K, 300, 1024, 513), (synth.Q4_K, 14336, 512, 1000), (synth.Q8_0, 4096, 2048, 1025), (synth.Q6_K, 1000, 2560, 777),
+                                       (synth.Q4_K, 2560, 2560, 2000), (synth.Q6_K, 257, 4096, 1537)])
+def test_long_prompts(fmt, N, K, M):
+    from brotensor_b200 import ops
+    Wh, xh = synth.make_blocks(fmt, N, K, seed=N + M), synth.make_activations(M, K, seed=M)
+    bh = synth.make_activations(1, N, seed=5).reshape(-1)
+    W, X, b = torch.from_numpy(Wh).cuda(), torch.from_numpy(xh).cuda(), torch.from_numpy(bh).cuda()
+    y = ops.gemm(fmt, W, X, N, bias=b)
+    assert torch.equal(y, ops.gemm(fmt, W, X, N, bias=b))
+    half = ops.gemm(fmt, W, X.half(), N, bias=b.half(), out_dtype=torch.float16)
+    rows = np.arange(0, N, max(1, N // 100))
+    want = oracle.cpu().matmul(fmt, Wh.reshape(N, -1)[rows].reshape(-1), xh, threads=16) + bh[None, rows]
+    cols = torch.from_numpy(rows).cuda()
+    assert oracle.rel_l2(y[:, cols].cpu().numpy(), want) < 2e-3
+    assert oracle.rel_l2(half[:, cols].float().cpu().numpy(), want) < 2e-3
+    try:
+        ops.set_option("gemm_pair", 0)
+        one = ops.gemm(fmt, W, X, N, bias=b)
+    finally:
+        ops.set_option("gemm_pair", 1)
+    assert oracle.rel_l2(y.cpu().numpy(), one.cpu().numpy()) < 1e-5  # the order of the FP32 additions of a split K alone
+    assert ops.device_status() == 0
