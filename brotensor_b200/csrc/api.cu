@@ -40,6 +40,10 @@ int launch_gemv_xr(int fmt, const void* W, const void* X, int x_dtype, const voi
                    int sms, int* status, cudaStream_t st, bool* taken);
 int launch_gemv_i8(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
                    int sms, int* status, cudaStream_t st, bool* taken);
+int launch_gemv_hm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
+                   int sms, cudaStream_t st, bool* taken);
+void hm_set_enabled(int v);
+int hm_get_enabled();
 void i8_set_enabled(int v);
 int i8_get_enabled();
 void xr_set_enabled(int v);
@@ -262,6 +266,29 @@ static int gemv_streaming(DevInfo* d, int fmt, const void* W, const void* X, int
     return B200Q_OK;
 }
 
+// Which decode calls go to the two raw-quant MMA kernels (gemv_hm.cu: 16-bit activations; gemv_mb.cu: any). Both do a call of
+// few weight rows per SM in little more than a launch, whatever M is, and stream long matrices at half the memory's
+// rate, so the lines lie where the older kernels' times cross theirs (us, old -> gemv_hm, FP16, overlapped launches):
+//   Q4_K   M = 2: 1024 x 4096 4.6 -> 3.7, 6912 x 2560 7.7 -> 6.3, 4096 x 14336 15.9 -> 17.9, 14336 x 4096 12.5 -> 19.1
+//          M = 6: 4096 x 4096 10.6 -> 6.5, 4096 x 14336 49 -> 18.5, 2560 x 6912 22 -> 9.6, 14336 x 4096 (integer MMA) 18.1 -> 19.0
+//   Q6_K   M = 2: 1024 x 4096 4.9 -> 4.3, 4096 x 4096 7.7 -> 8.3; M = 6: 10.3 -> 8.7, 4096 x 14336 43 -> 25, 14336 x 4096 22 -> 25
+//   Q8_0   M = 2: 4096 x 4096 10.9 -> 7.7, 4096 x 14336 19.8 -> 21.6; M = 6: 11.4 -> 7.9, 43.6 -> 22, 14336 x 4096 18.8 -> 21.9
+// Rows of Q6_K that are not whole runs of eight blocks, Q5_K and Q4_0 had the plain-load kernel (2560 x 6912, M = 1: 20.8 -> 11.6,
+// 24.8 -> 10.2, 19.8 -> 8.0); from M = 1, 2 and many rows gemv_mb is the faster of the two for the 4- and 5-bit formats (14336 x 4096
+// Q5_K 21.6 against 17.1, 32003 x 2560 Q6_K 33.3 against 27.3, 32000 x 4096 Q4_0 32.8 against 30.8).
+static bool hm_wanted(int fmt, int x_dtype, int M, int N, int K) {
+    if (x_dtype == B200Q_DT_F32) return false;
+    if (hm_get_enabled() == 2) return true;
+    const bool few = N <= 8192;
+    switch (fmt) {
+        case kQ5_K: return M > 2 || few;
+        case kQ4_0: return M > 2 || N <= 16384;
+        case kQ4_K: return M == 2 ? K <= 4096 && (long long)N * K <= 18000000 : M > 2 && (few || (M >= 4 && K != 2048 && K != 4096));
+        case kQ6_K: return K % kQ6RunElems != 0 ? M > 2 || few : M >= 4 ? few : M >= 2 && N <= 2048;
+        case kQ8_0: return M >= 2 && (few ? M > 2 || K <= 8192 : M > 2 && K != 2048 && K != 4096 && N <= 16384);
+    }
+    return false;
+}
 int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M,
                int N, int K, void* stream) {
     if (int rc = check_linear_args("gemv", fmt, W, X, x_dtype, Y, y_dtype, M, N, K)) return rc;
@@ -270,6 +297,11 @@ int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* b
     DevInfo* d;
     if (int rc = dev_info(&d)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (g_opt_gemv_path == 0 && hm_wanted(fmt, x_dtype, M, N, K)) {
+        bool taken = false;
+        if (int rc = launch_gemv_hm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, st, &taken)) return rc;
+        if (taken) return B200Q_OK;
+    }
     if (!streaming_fmt(fmt)) return launch_gemv_simple(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
     // 0 = automatic, 1 = plain-load kernel, 2 = warp-MMA streaming kernel, 3 = integer-dot streaming kernel
     if (g_opt_gemv_path == 0) {
@@ -439,12 +471,17 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
     DevInfo* d;
     if (int rc = dev_info(&d)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // Up to sixteen rows of 16-bit activations of a matrix of few rows: two passes of the small-batch GEMV (4096 x 4096 Q4_K 13 us
+    // against 20, 2560 x 6912 Q4_K 20 against 31, 4096 x 14336 Q5_K 42 against 60 of the kernels below).
+    const bool two_passes = g_opt_gemm_path == 0 && g_opt_gemv_path == 0 && M > 8 && M <= 16 && N <= 8192 && K % 256 == 0 && fmt != kQ6_KP &&
+                            hm_get_enabled() && hm_wanted(fmt, x_dtype, 8, N, K) &&
+                            (fmt == kQ6_K || aligned(W, 16));
     // Nine to sixteen rows: the tensor-core GEMM's producers decode the whole matrix for however few tokens
     // (14336 x 4096: 46-48 us for any M up to 32), two passes of the small-batch GEMV on the integer tensor
     // cores take 28-30 us (Q4_K, Q8_0; 4096 x 4096: 14-15 against 18-20), and for Q6_K from 8192 rows two
     // passes of the warp-MMA GEMV 53-55 against 67. From 24 rows the GEMM is the faster one.
-    if (g_opt_gemm_path == 0 && M > 8 && M <= 16 && K <= 4096 &&
-        (((fmt == kQ4_K || fmt == kQ8_0) && (K == 2048 || K == 4096) && i8_get_enabled()) || (fmt == kQ6_K && N >= 8192))) {
+    if (two_passes || (g_opt_gemm_path == 0 && M > 8 && M <= 16 && K <= 4096 &&
+        (((fmt == kQ4_K || fmt == kQ8_0) && (K == 2048 || K == 4096) && i8_get_enabled()) || (fmt == kQ6_K && N >= 8192)))) {
         const size_t xs = (size_t)dt_size(x_dtype) * K, ys = (size_t)dt_size(y_dtype) * N;
         for (int m0 = 0; m0 < M; m0 += 8) {
             const int mm = M - m0 < 8 ? M - m0 : 8;
@@ -452,7 +489,7 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
                                     static_cast<char*>(Y) + ys * m0, y_dtype, mm, N, K, stream))
                 return rc;
         }
-        d->tc_calls[fmt_slot(fmt)].fetch_add(1);  // mma.sync on the tensor cores, int8 or FP16
+        if (fmt_slot(fmt) >= 0) d->tc_calls[fmt_slot(fmt)].fetch_add(1);  // mma.sync on the tensor cores, int8 or 16-bit
         return B200Q_OK;
     }
     if (g_opt_gemm_path != 1) {
@@ -526,6 +563,7 @@ int b200q_set_option(const char* key, int value) {
     else if (!strcmp(key, "gemv_lean")) dp_set_lean(value);
     else if (!strcmp(key, "gemv_xr")) xr_set_enabled(value);
     else if (!strcmp(key, "gemv_i8")) i8_set_enabled(value);
+    else if (!strcmp(key, "gemv_hm")) hm_set_enabled(value);
     else if (!strcmp(key, "gemv_step_fill")) dp_set_step_fill(value);
     else return fail(B200Q_ERR_BAD_ARG, "set_option: unknown key '%s'", key);
     return B200Q_OK;
@@ -541,6 +579,7 @@ int b200q_get_option(const char* key, int* out) {
     else if (!strcmp(key, "gemv_groups")) *out = dp_get_groups();
     else if (!strcmp(key, "gemv_xr")) *out = xr_get_enabled();
     else if (!strcmp(key, "gemv_i8")) *out = i8_get_enabled();
+    else if (!strcmp(key, "gemv_hm")) *out = hm_get_enabled();
     else if (!strcmp(key, "gemv_tile_pairs")) *out = dp_get_tile_pairs();
     else if (!strcmp(key, "gemm_pair")) *out = gemm_get_pair();
     else if (!strcmp(key, "gemm_split")) *out = gemm_get_split();

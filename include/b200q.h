@@ -287,10 +287,12 @@ int b200q_device_status(int* status_out);
  *                 decode GEMV only, 2 = the tcgen05 GEMM or an error
  *   "gemm_pair"   0 = one-CTA tcgen05 kernel, otherwise the CTA-pair kernel (default)
  *   "gemm_split"  0 = never split K; 1 (default) = where it shortens the call, matrices of few row tiles
- *                 (N <= 9472) have their k-blocks split over up to eight CTA pairs, partial sums added in a
+ *                 have their k-blocks split over up to eight CTA pairs, partial sums added in a
  *                 fixed order by a second kernel (b200q_gemm_workspace_bytes() grows accordingly)
  *   "gemv_xr"     Q4_K / Q6_K, one activation row, K <= 4096: 1 = the activation-resident kernel where it is the
  *                 faster one (default), 2 = for every such call, 0 = never
+ *   "gemv_hm"     FP16 / BF16 activations, 1..8 rows: 1 = the raw-quant tensor-core kernel where it is the faster one (default),
+ *                 2 = for every such call, 0 = never
  *   "gemv_i8"     Q8_0 / Q4_K, 2..8 activation rows, K = 2048 / 4096: 1 = the integer tensor-core kernel where it is
  *                 the faster one (default), 2 = for every such call, 0 = never
  *   "gemv_lean"   0 = never take the trimmed instantiation of the integer-dot kernel (FP32 in and out, no bias)

@@ -1,0 +1,91 @@
+"""The kernel that multiplies raw quants on the warp-level tensor-core instructions, csrc/gemv_hm.cu (16-bit activations, 1..8 rows), against
+the oracle's 64-bit sums. Nothing in it is rounded below
+FP32: exact products, sums of a few hundred FP32 terms (at most sqrt(K / 32 + 16) * 2^-24 < 2e-6 over a row for K <= 14336), so that is the bound.
+Sizes: one row, ragged tiles of 16, fewer rows than SMs, several row tiles per CTA, several passes over a CTA's rows, K of one block, of
+an odd number of blocks (Q6_K rows that start on any even byte) and of more blocks than a CTA has warps."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle
+from brotensor_b200 import synth
+
+FMTS = [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0, synth.Q4_0]
+SHAPES = [(1, 256), (15, 512), (37, 768), (300, 6912), (2373, 1024), (40, 14336), (20000, 256)]
+DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
+
+
+@pytest.fixture
+def ops_raw():
+    from brotensor_b200 import ops
+    yield ops
+    for key in ("gemv_hm",):
+        ops.set_option(key, 1)
+    ops.set_option("pdl", 0)
+    assert ops.device_status() == 0
+
+
+def _operands(fmt, N, K, M, dtype):
+    Wh = synth.make_blocks(fmt, N, K, seed=N + K)
+    x = torch.from_numpy(synth.make_activations(M, K, seed=M + K)).to(DT[dtype])
+    b = torch.from_numpy(synth.make_activations(1, N, seed=5).reshape(-1)).to(DT[dtype])
+    want = oracle.cpu().matmul(fmt, Wh, x.float().numpy(), bias=b.float().numpy(), threads=8, want_f64=True)[1]
+    return torch.from_numpy(Wh).cuda(), x.cuda(), b.cuda(), want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", SHAPES)
+@pytest.mark.parametrize("fmt", FMTS)
+def test_decode_rows(fmt, N, K, ops_raw):
+    ops = ops_raw
+    for M, dtype in ((1, "f16"), (2, "bf16"), (3, "f32"), (5, "bf16"), (7, "f32"), (8, "bf16"), (8, "f16")):
+        W, x, b, want = _operands(fmt, N, K, M, dtype)
+        for kernel in ("gemv_hm",):
+            if kernel == "gemv_hm" and dtype == "f32":
+                continue
+            ops.set_option("gemv_hm", 2 if kernel == "gemv_hm" else 0)
+            y = ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32)
+            assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (kernel, M, dtype)
+            assert torch.equal(y, ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32))  # fixed order of additions
+            for early in (-1, 1):
+                ops.set_option("pdl", early)
+                assert torch.equal(y, ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32))
+            ops.set_option("pdl", 0)
+            half = ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float16)
+            assert torch.equal(half, y.half())  # one rounding of the same sums
+
+
+@pytest.mark.gpu
+def test_weights_on_two_byte_boundaries(ops_raw):
+    """Q6_K rows may start anywhere; the other formats' unaligned weights keep going to the plain kernel."""
+    ops = ops_raw
+    for fmt, shift in ((synth.Q6_K, 2), (synth.Q6_K, 14), (synth.Q8_0, 2), (synth.Q4_0, 6), (synth.Q5_K, 4)):
+        N, K = 77, 1280
+        for M, dtype in ((1, "f16"), (4, "bf16")):
+            W, x, b, want = _operands(fmt, N, K, M, dtype)
+            buf = torch.zeros(W.numel() + 64, dtype=torch.uint8, device="cuda")
+            moved = buf[shift:shift + W.numel()]
+            moved.copy_(W.reshape(-1))
+            y = ops.linear(fmt, moved, x, N, bias=b, out_dtype=torch.float32)
+            assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", FMTS)
+def test_activations_that_are_not_finite(fmt, ops_raw):
+    """Infinities and NaN give what FP32 arithmetic on the decoded weights gives."""
+    ops = ops_raw
+    N, K = 200, 1024
+    W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=3)).cuda()
+    for M, dtype in ((3, "f16"), (3, "bf16")):
+        for value in (float("inf"), float("-inf"), float("nan")):
+            x = torch.from_numpy(synth.make_activations(M, K, seed=4)).to(DT[dtype]).cuda()
+            x[1, 77] = value
+            y = ops.linear(fmt, W, x, N, out_dtype=torch.float32)
+            ops.set_option("gemv_path", 1)
+            want = torch.cat([ops.gemv(fmt, W, x[i:i + 1], N, out_dtype=torch.float32) for i in range(M)])
+            ops.set_option("gemv_path", 0)
+            assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+            ok = torch.isfinite(want)
+            assert torch.allclose(y[ok], want[ok], rtol=1e-4, atol=1e-4)
