@@ -40,10 +40,19 @@ int launch_gemv_xr(int fmt, const void* W, const void* X, int x_dtype, const voi
                    int sms, int* status, cudaStream_t st, bool* taken);
 int launch_gemv_i8(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
                    int sms, int* status, cudaStream_t st, bool* taken);
+int launch_gemv_mb(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
+                   int sms, int* status, cudaStream_t st, bool* taken);
+void mb_set_enabled(int v);
 int launch_gemv_hm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
                    int sms, cudaStream_t st, bool* taken);
 void hm_set_enabled(int v);
 int hm_get_enabled();
+size_t gemm_mm_workspace_bytes(int fmt, int x_dtype, int M, int N, int K);
+int launch_gemm_mm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
+                   void* ws, size_t ws_bytes, int sms, cudaStream_t st, bool* taken);
+void mm_set_enabled(int v);
+int mm_get_enabled();
+int mb_get_enabled();
 void i8_set_enabled(int v);
 int i8_get_enabled();
 void xr_set_enabled(int v);
@@ -289,6 +298,11 @@ static bool hm_wanted(int fmt, int x_dtype, int M, int N, int K) {
     }
     return false;
 }
+static bool mb_wanted(int fmt, int M, int N, int K) {
+    if (mb_get_enabled() == 2) return true;
+    return !streaming_fmt(fmt) || (fmt == kQ6_K && K % kQ6RunElems != 0);
+}
+
 int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M,
                int N, int K, void* stream) {
     if (int rc = check_linear_args("gemv", fmt, W, X, x_dtype, Y, y_dtype, M, N, K)) return rc;
@@ -300,6 +314,11 @@ int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* b
     if (g_opt_gemv_path == 0 && hm_wanted(fmt, x_dtype, M, N, K)) {
         bool taken = false;
         if (int rc = launch_gemv_hm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, st, &taken)) return rc;
+        if (taken) return B200Q_OK;
+    }
+    if (g_opt_gemv_path == 0 && mb_wanted(fmt, M, N, K)) {
+        bool taken = false;
+        if (int rc = launch_gemv_mb(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->status, st, &taken)) return rc;
         if (taken) return B200Q_OK;
     }
     if (!streaming_fmt(fmt)) return launch_gemv_simple(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
@@ -459,9 +478,13 @@ int b200q_gemv_shard_topk(int fmt, const void* W_shard, const void* x, int x_dty
                            peer_out, peer_cand, state, k, top_val, top_idx, stream);
 }
 
+// Q5_K and Q4_0 have no tcgen05 form (an FP16 weight would be less than they are multiplied with).
+static bool mm_wanted(int fmt, int M) { return M > 8 && mm_get_enabled() && !streaming_fmt(fmt); }
+
 size_t b200q_gemm_workspace_bytes(int fmt, int x_dtype, int M, int N, int K) {
     if (!b200q_block_elems(fmt) || M <= 0 || N <= 0 || K <= 0) return 0;
-    return gemm_tc_workspace_bytes(fmt, x_dtype, M, N, K);
+    const size_t tc = gemm_tc_workspace_bytes(fmt, x_dtype, M, N, K), mm = mm_wanted(fmt, M) ? gemm_mm_workspace_bytes(fmt, x_dtype, M, N, K) : 0;
+    return tc > mm ? tc : mm;
 }
 
 int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M,
@@ -476,6 +499,14 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
     const bool two_passes = g_opt_gemm_path == 0 && g_opt_gemv_path == 0 && M > 8 && M <= 16 && N <= 8192 && K % 256 == 0 && fmt != kQ6_KP &&
                             hm_get_enabled() && hm_wanted(fmt, x_dtype, 8, N, K) &&
                             (fmt == kQ6_K || aligned(W, 16));
+    if (!two_passes && g_opt_gemm_path == 0 && mm_wanted(fmt, M)) {
+        bool taken = false;
+        if (int rc = launch_gemm_mm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, ws, ws_bytes, d->sms, st, &taken)) return rc;
+        if (taken) {
+            if (fmt_slot(fmt) >= 0) d->tc_calls[fmt_slot(fmt)].fetch_add(1);
+            return B200Q_OK;
+        }
+    }
     // Nine to sixteen rows: the tensor-core GEMM's producers decode the whole matrix for however few tokens
     // (14336 x 4096: 46-48 us for any M up to 32), two passes of the small-batch GEMV on the integer tensor
     // cores take 28-30 us (Q4_K, Q8_0; 4096 x 4096: 14-15 against 18-20), and for Q6_K from 8192 rows two
@@ -563,7 +594,9 @@ int b200q_set_option(const char* key, int value) {
     else if (!strcmp(key, "gemv_lean")) dp_set_lean(value);
     else if (!strcmp(key, "gemv_xr")) xr_set_enabled(value);
     else if (!strcmp(key, "gemv_i8")) i8_set_enabled(value);
+    else if (!strcmp(key, "gemv_mb")) mb_set_enabled(value);
     else if (!strcmp(key, "gemv_hm")) hm_set_enabled(value);
+    else if (!strcmp(key, "gemm_mm")) mm_set_enabled(value);
     else if (!strcmp(key, "gemv_step_fill")) dp_set_step_fill(value);
     else return fail(B200Q_ERR_BAD_ARG, "set_option: unknown key '%s'", key);
     return B200Q_OK;
@@ -579,7 +612,9 @@ int b200q_get_option(const char* key, int* out) {
     else if (!strcmp(key, "gemv_groups")) *out = dp_get_groups();
     else if (!strcmp(key, "gemv_xr")) *out = xr_get_enabled();
     else if (!strcmp(key, "gemv_i8")) *out = i8_get_enabled();
+    else if (!strcmp(key, "gemv_mb")) *out = mb_get_enabled();
     else if (!strcmp(key, "gemv_hm")) *out = hm_get_enabled();
+    else if (!strcmp(key, "gemm_mm")) *out = mm_get_enabled();
     else if (!strcmp(key, "gemv_tile_pairs")) *out = dp_get_tile_pairs();
     else if (!strcmp(key, "gemm_pair")) *out = gemm_get_pair();
     else if (!strcmp(key, "gemm_split")) *out = gemm_get_split();

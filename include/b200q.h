@@ -293,6 +293,9 @@ int b200q_device_status(int* status_out);
  *                 faster one (default), 2 = for every such call, 0 = never
  *   "gemv_hm"     FP16 / BF16 activations, 1..8 rows: 1 = the raw-quant tensor-core kernel where it is the faster one (default),
  *                 2 = for every such call, 0 = never
+ *   "gemv_mb"     Q5_K, Q4_0, Q6_K, 1..8 rows: 1 = the integer tensor-core kernel for calls that would else go to the plain-load
+ *                 kernel (default), 2 = for every such call "gemv_hm" leaves, 0 = never
+ *   "gemm_mm"     Q5_K, Q4_0 from 9 rows: 1 = the warp-level tensor-core GEMM (default), 0 = passes of the decode GEMV
  *   "gemv_i8"     Q8_0 / Q4_K, 2..8 activation rows, K = 2048 / 4096: 1 = the integer tensor-core kernel where it is
  *                 the faster one (default), 2 = for every such call, 0 = never
  *   "gemv_lean"   0 = never take the trimmed instantiation of the integer-dot kernel (FP32 in and out, no bias)

@@ -1,5 +1,5 @@
-"""The kernel that multiplies raw quants on the warp-level tensor-core instructions, csrc/gemv_hm.cu (16-bit activations, 1..8 rows), against
-the oracle's 64-bit sums. Nothing in it is rounded below
+"""The kernels that multiply raw quants on the warp-level tensor-core instructions - csrc/gemv_hm.cu (16-bit activations, 1..8 rows), csrc/gemv_mb.cu
+(Q5_K, Q4_0, Q6_K with any activations, 1..8 rows) and csrc/gemm_mm.cu (Q5_K, Q4_0, from nine tokens) - against the oracle's 64-bit sums. Nothing in them is rounded below
 FP32: exact products, sums of a few hundred FP32 terms (at most sqrt(K / 32 + 16) * 2^-24 < 2e-6 over a row for K <= 14336), so that is the bound.
 Sizes: one row, ragged tiles of 16, fewer rows than SMs, several row tiles per CTA, several passes over a CTA's rows, K of one block, of
 an odd number of blocks (Q6_K rows that start on any even byte) and of more blocks than a CTA has warps."""
@@ -20,7 +20,7 @@ DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
 def ops_raw():
     from brotensor_b200 import ops
     yield ops
-    for key in ("gemv_hm",):
+    for key in ("gemv_hm", "gemv_mb", "gemm_mm"):
         ops.set_option(key, 1)
     ops.set_option("pdl", 0)
     assert ops.device_status() == 0
@@ -41,10 +41,13 @@ def test_decode_rows(fmt, N, K, ops_raw):
     ops = ops_raw
     for M, dtype in ((1, "f16"), (2, "bf16"), (3, "f32"), (5, "bf16"), (7, "f32"), (8, "bf16"), (8, "f16")):
         W, x, b, want = _operands(fmt, N, K, M, dtype)
-        for kernel in ("gemv_hm",):
+        for kernel in ("gemv_hm", "gemv_mb"):
             if kernel == "gemv_hm" and dtype == "f32":
                 continue
             ops.set_option("gemv_hm", 2 if kernel == "gemv_hm" else 0)
+            ops.set_option("gemv_mb", 2)
+            if kernel == "gemv_mb" and fmt in (synth.Q4_K, synth.Q8_0):
+                continue
             y = ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32)
             assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (kernel, M, dtype)
             assert torch.equal(y, ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32))  # fixed order of additions
@@ -57,12 +60,26 @@ def test_decode_rows(fmt, N, K, ops_raw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K", SHAPES)
+@pytest.mark.parametrize("fmt", [synth.Q5_K, synth.Q4_0])
+def test_a_few_dozen_tokens(fmt, N, K, ops_raw):
+    ops = ops_raw
+    for M, dtype in ((9, "f16"), (17, "f32"), (33, "bf16"), (64, "f16"), (65, "f32"), (131, "f16")):
+        if N * K * M > 4e8:
+            continue
+        W, x, b, want = _operands(fmt, N, K, M, dtype)
+        y = ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32)
+        assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (M, dtype)
+        assert torch.equal(y, ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32))
+
+
+@pytest.mark.gpu
 def test_weights_on_two_byte_boundaries(ops_raw):
     """Q6_K rows may start anywhere; the other formats' unaligned weights keep going to the plain kernel."""
     ops = ops_raw
     for fmt, shift in ((synth.Q6_K, 2), (synth.Q6_K, 14), (synth.Q8_0, 2), (synth.Q4_0, 6), (synth.Q5_K, 4)):
         N, K = 77, 1280
-        for M, dtype in ((1, "f16"), (4, "bf16")):
+        for M, dtype in ((1, "f16"), (4, "f32"), (20, "f16")):
             W, x, b, want = _operands(fmt, N, K, M, dtype)
             buf = torch.zeros(W.numel() + 64, dtype=torch.uint8, device="cuda")
             moved = buf[shift:shift + W.numel()]
@@ -78,7 +95,10 @@ def test_activations_that_are_not_finite(fmt, ops_raw):
     ops = ops_raw
     N, K = 200, 1024
     W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=3)).cuda()
-    for M, dtype in ((3, "f16"), (3, "bf16")):
+    plain = fmt in (synth.Q5_K, synth.Q4_0)  # formats whose every form sums in FP32
+    for M, dtype in ((3, "f16"), (3, "f32"), (20, "f16"), (20, "f32")):
+        if not plain and (M > 8 or (dtype == "f32" and fmt != synth.Q6_K)):
+            continue
         for value in (float("inf"), float("-inf"), float("nan")):
             x = torch.from_numpy(synth.make_activations(M, K, seed=4)).to(DT[dtype]).cuda()
             x[1, 77] = value
@@ -89,3 +109,19 @@ def test_activations_that_are_not_finite(fmt, ops_raw):
             assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
             ok = torch.isfinite(want)
             assert torch.allclose(y[ok], want[ok], rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.gpu
+def test_magnitudes_that_fp16_cannot_hold(ops_raw):
+    """FP32 and BF16 activations far outside FP16's range are scaled, not rounded away."""
+    ops = ops_raw
+    fmt, N, K = synth.Q5_K, 96, 2048
+    Wh = synth.make_blocks(fmt, N, K, seed=8)
+    W = torch.from_numpy(Wh).cuda()
+    for M in (2, 6, 24):
+        for dtype in ("f32", "bf16"):
+            for scale in (1e-25, 1e-6, 1e6, 1e25):
+                x = (torch.from_numpy(synth.make_activations(M, K, seed=9)) * scale).to(DT[dtype])
+                want = oracle.cpu().matmul(fmt, Wh, x.float().numpy(), threads=8, want_f64=True)[1]
+                y = ops.linear(fmt, W, x.cuda(), N, out_dtype=torch.float32).cpu().numpy()
+                assert oracle.rel_l2(y / np.float32(scale), want / scale) < 2e-6
