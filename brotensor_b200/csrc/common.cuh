@@ -371,12 +371,18 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void prefetch_l2_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Loads of what the stream's predecessor may have written, for kernels that start before it has finished: ordinary
 // coherent loads that stay behind griddepcontrol.wait (the read-only path promises data that nobody
 // writes while the kernel lives, and its loads may be moved).
 __device__ __forceinline__ uint4 ld_dep_u4(const void* p) {
     uint4 v;
     asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_dep_u16(const void* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint2 ld_dep_u2(const void* p) {

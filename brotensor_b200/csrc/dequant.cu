@@ -104,11 +104,6 @@ __global__ void __launch_bounds__(256) dequant_k_kernel(const uint8_t* W, OT* ou
 // each of the half's four 32-element quarters - so four runs of stores, and the loads and the scale
 // work of the generic path are shared by four times as many outputs. Blocks are 2-byte aligned only;
 // all loads are 16-bit pairs. d * sc * (q - 32) is exact in FP32 (11 + 7 + 6 bits), one rounding to the output type.
-__device__ __forceinline__ uint32_t ld_dep_u16(const void* p) {
-    unsigned short v;
-    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-    return v;
-}
 __device__ __forceinline__ uint32_t ld_dep_u32_a2(const uint8_t* p) { return ld_dep_u16(p) | (ld_dep_u16(p + 2) << 16); }
 template <bool RUNS, typename OT>  // RUNS: the layout regrouped by field in runs of eight blocks (16-byte aligned fields)
 __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* W, OT* out, long long total_units, int units_per_row, int row_bytes, int K) {

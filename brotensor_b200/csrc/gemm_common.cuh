@@ -32,9 +32,11 @@ struct GemmParams {
 // ---- activation pre-pass ---------------------------------------------------------------
 // Xp[kb][t][c ^ (t & 7)] (16-byte chunks) = FP16(X[t][64*kb + 8*c .. +8]); rows t >= M are zero.
 template <typename XT>
-__global__ void __launch_bounds__(256) gemm_xprep_kernel(const XT* __restrict__ X, uint4* __restrict__ Xp, int M,
+__global__ void __launch_bounds__(256) gemm_xprep_kernel(const XT* X, uint4* Xp, int M,
                                                          int tok_pad, int K) {
     const long long total = (long long)(K / 64) * tok_pad * 8;
+    grid_dep_launch();
+    grid_dep_wait();  // the activations, and the workspace that the launch before may still read
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(idx & 7);
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(256) gemm_xprep_kernel(const XT* __restrict__ 
         if (t < M) {
             const XT* src = X + (size_t)t * K + (size_t)kb * 64 + c * 8;
             if constexpr (sizeof(XT) == 4) {
-                const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+                const float4 a = ld_dep_f4(src), b = ld_dep_f4(src + 4);
                 o.h[0] = __float2half_rn(a.x); o.h[1] = __float2half_rn(a.y); o.h[2] = __float2half_rn(a.z); o.h[3] = __float2half_rn(a.w);
                 o.h[4] = __float2half_rn(b.x); o.h[5] = __float2half_rn(b.y); o.h[6] = __float2half_rn(b.z); o.h[7] = __float2half_rn(b.w);
             } else {
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(256) gemm_xprep_kernel(const XT* __restrict__ 
                     uint4 q;
                     XT e[8];
                 } in;
-                in.q = __ldg(reinterpret_cast<const uint4*>(src));
+                in.q = ld_dep_u4(src);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) o.h[k] = __float2half_rn(to_f32<XT>(in.e[k]));
             }

@@ -300,10 +300,10 @@ int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const voi
         long long blocks = (total + 255) / 256;
         if (blocks > 148LL * 16) blocks = 148LL * 16;
         uint4* xp = static_cast<uint4*>(ws);
-        if (x_dtype == B200Q_DT_F32) gemm_xprep_kernel<float><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float*>(X), xp, M, tok_total, K);
-        else if (x_dtype == B200Q_DT_F16) gemm_xprep_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const __half*>(X), xp, M, tok_total, K);
-        else gemm_xprep_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(X), xp, M, tok_total, K);
-        B200Q_CUDA_TRY(cudaGetLastError());
+        const bool overlap = pdl_option() >= 0;
+        if (x_dtype == B200Q_DT_F32) B200Q_CUDA_TRY(launch_dep(overlap, gemm_xprep_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const float*>(X), xp, M, tok_total, K));
+        if (x_dtype == B200Q_DT_F16) B200Q_CUDA_TRY(launch_dep(overlap, gemm_xprep_kernel<__half>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const __half*>(X), xp, M, tok_total, K));
+        if (x_dtype == B200Q_DT_BF16) B200Q_CUDA_TRY(launch_dep(overlap, gemm_xprep_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(X), xp, M, tok_total, K));
     }
     const int ysz = y_dtype == B200Q_DT_F32 ? 4 : 2;
     if (g_gemm_pair != 0)

@@ -230,10 +230,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
         tmem_alloc2(smem_u32(&tmem_base_slot), tmem_cols);
         tmem_relinquish2();
     }
+    // The set-up overlaps the predecessor (the activation pre-pass); its results, and weights that something before it may have
+    // written, are read behind griddepcontrol.wait. The L2 hears about the rows' first lines meanwhile.
+    grid_dep_launch();
+    if (warp >= kPairCtrlWarps) {
+        const int r = min(row0 + (warp & 3) * 32 + lane, p.N - 1);
+        prefetch_l2_line(p.W + (size_t)r * p.row_bytes + (size_t)blockIdx.y * p.w_split_bytes + 128 * ((warp - kPairCtrlWarps) >> 2));
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // the peer's barriers exist before anything arrives on them
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = tmem_base_slot;
     const uint32_t b_base = sbase + (uint32_t)(p.n_a * kGemmRows * 128);  // A ring first, then the slab ring
 
@@ -328,9 +336,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
         for (int i = 0; i < 5; ++i) cur[i] = nxt[i] = make_uint4(0, 0, 0, 0);
         auto q4_load = [&](int b, uint4 (&dst)[5]) {
             const uint4* src = reinterpret_cast<const uint4*>(rowp + (size_t)b * 144);
-            dst[0] = __ldg(src);
+            dst[0] = ld_dep_u4(src);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) dst[1 + i] = __ldg(src + 1 + 2 * i + H);
+            for (int i = 0; i < 4; ++i) dst[1 + i] = ld_dep_u4(src + 1 + 2 * i + H);
         };
         if constexpr (FMT == kQ4_K) q4_load(0, nxt);
         // Q8_0: eight blocks (256 k, 272 bytes = 17 x 16) form a 16-byte aligned chunk. The thread's
@@ -340,7 +348,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
         auto q8_load = [&](int kbb, uint4 (&dst)[3]) {
             const uint4* src = reinterpret_cast<const uint4*>(rowp + (size_t)(kbb >> 2) * 272) + 4 * (kbb & 3) + 2 * H;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
+            for (int i = 0; i < 3; ++i) dst[i] = ld_dep_u4(src + i);
         };
 #pragma unroll
         for (int i = 0; i < 3; ++i) c8[i] = c8n[i] = make_uint4(0, 0, 0, 0);
@@ -365,11 +373,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
                 const int s = blk & 7;
                 const uint4* al = reinterpret_cast<const uint4*>(run + s * 128 + 64 * grp + 32 * H);
                 const uint4* ah = reinterpret_cast<const uint4*>(run + 1024 + s * 64 + 32 * grp);
-                L[0] = __ldg(al); L[1] = __ldg(al + 1);
-                Hh[0] = __ldg(ah); Hh[1] = __ldg(ah + 1);
-                S = (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(run + 1536 + s * 16 + grp * 8 + H * 2)) |
-                    (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(run + 1536 + s * 16 + grp * 8 + 4 + H * 2)) << 16;
-                D = __ldg(reinterpret_cast<const unsigned short*>(run + 1664 + 2 * s));
+                L[0] = ld_dep_u4(al); L[1] = ld_dep_u4(al + 1);
+                Hh[0] = ld_dep_u4(ah); Hh[1] = ld_dep_u4(ah + 1);
+                S = ld_dep_u16(run + 1536 + s * 16 + grp * 8 + H * 2) |
+                    ld_dep_u16(run + 1536 + s * 16 + grp * 8 + 4 + H * 2) << 16;
+                D = ld_dep_u16(run + 1664 + 2 * s);
                 F = 0;
                 return;
             }
@@ -377,12 +385,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
             F = (uint32_t)(reinterpret_cast<uintptr_t>(b0) & 15u);
             const uint4* al = reinterpret_cast<const uint4*>(b0 - F);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) L[i] = __ldg(al + 4 * grp + 2 * H + i);
+            for (int i = 0; i < 3; ++i) L[i] = ld_dep_u4(al + 4 * grp + 2 * H + i);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) Hh[i] = __ldg(al + 8 + 2 * grp + i);
-            S = (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(b0 + 192 + grp * 8 + H * 2)) |
-                (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(b0 + 192 + grp * 8 + 4 + H * 2)) << 16;
-            D = __ldg(reinterpret_cast<const unsigned short*>(b0 + 208));
+            for (int i = 0; i < 3; ++i) Hh[i] = ld_dep_u4(al + 8 + 2 * grp + i);
+            S = ld_dep_u16(b0 + 192 + grp * 8 + H * 2) |
+                ld_dep_u16(b0 + 192 + grp * 8 + 4 + H * 2) << 16;
+            D = ld_dep_u16(b0 + 208);
         };
 #pragma unroll
         for (int i = 0; i < 3; ++i) l6[i] = h6[i] = l6n[i] = h6n[i] = make_uint4(0, 0, 0, 0);
@@ -544,21 +552,25 @@ static int launch_pair_fmt(const PairParams& p, size_t smem, cudaStream_t st) {
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_option() >= 0 ? 2 : 1;
     B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
     return B200Q_OK;
 }
 
 // Y[t][n] = bias[n] + part[0][t][n] + part[1][t][n] + ... in that order (the same on every run), four
 // neighbouring n per thread.
-__global__ void __launch_bounds__(256) gemm_split_reduce_kernel(const float* __restrict__ part, int n_split, int tokens, int N,
-                                                                const void* __restrict__ bias, int bias_dtype, void* __restrict__ Y, int y_dtype) {
+__global__ void __launch_bounds__(256) gemm_split_reduce_kernel(const float* part, int n_split, int tokens, int N, const void* bias, int bias_dtype,
+                                                                void* Y, int y_dtype) {
+    grid_dep_launch();
+    grid_dep_wait();
     const size_t total = (size_t)tokens * N, quads = total / 4;  // N % 4 == 0 is checked by the caller
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (size_t)gridDim.x * blockDim.x) {
         const int n = (int)((4 * i) % (size_t)N);
@@ -644,8 +656,7 @@ int launch_gemm_pair(int fmt, const void* W, const uint8_t* Xp, int tok_stride, 
     const size_t quads = (size_t)tokens * N / 4;
     size_t blocks = (quads + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    gemm_split_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(ypart, p.n_split, tokens, N, bias, bias_dtype, Y, y_dtype);
-    B200Q_CUDA_TRY(cudaGetLastError());
+    B200Q_CUDA_TRY(launch_dep(pdl_option() >= 0, gemm_split_reduce_kernel, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const float*>(ypart), (int)p.n_split, tokens, N, bias, bias_dtype, Y, y_dtype));
     return B200Q_OK;
 }
 

@@ -276,8 +276,9 @@ int b200q_device_status(int* status_out);
  *                 3 = integer-dot streaming kernel (a forced path fails on shapes it does not take)
  *   "gemv_stages" ring depth of the streaming kernels (2..8); "gemv_stage_kb" stage size target;
  *   "gemv_grid"   CTA count (0 = one per SM)
- *   "pdl"         0 (default) = the one-row decode GEMVs start under programmatic dependent launch and touch global memory
- *                 once their predecessor has finished; 1 = their weights (which then must not be written by the
+ *   "pdl"         0 (default) = the one-row decode GEMVs, the raw-quant kernels, the prefill GEMM's three kernels and the wide
+ *                 decode kernels start under programmatic dependent launch and touch global memory once their
+ *                 predecessor has finished; 1 = their weights (which then must not be written by the
  *                 launch before them in the stream) are read ahead of that; negative = plain launches
  *   "gemv_groups" pipelines per CTA of the integer-dot kernel (1 or 2); "gemv_tile_pairs" 2 = prefer
  *                 one pipeline with 32-row tiles; "gemv_split_full" (Q6_K only) -1 = automatic, 0 = one full

@@ -17,13 +17,15 @@ def ops_pdl():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("fmt,N,K,M", [(synth.Q4_K, 14336, 4096, 1), (synth.Q4_K, 4096, 4096, 1), (synth.Q4_K, 1024, 2560, 2), (synth.Q4_K, 4096, 4096, 6),
-                                       (synth.Q6_K, 4096, 14336, 1), (synth.Q6_K, 4096, 4096, 6), (synth.Q8_0, 4096, 4096, 3)])
+                                       (synth.Q6_K, 4096, 14336, 1), (synth.Q6_K, 4096, 4096, 6), (synth.Q8_0, 4096, 4096, 3), (synth.Q5_K, 3000, 2560, 1),
+                                       (synth.Q4_0, 700, 1024, 20), (synth.Q4_K, 1024, 4096, 40), (synth.Q6_K, 300, 8192, 17), (synth.Q8_0, 600, 2048, 600)])
 def test_predecessor_writes_the_operands(fmt, N, K, M, ops_pdl):
     ops = ops_pdl
     Ws = [torch.from_numpy(synth.make_blocks(fmt, N, K, seed=s)).cuda() for s in (1, 2)]
     xs = [torch.from_numpy(synth.make_activations(M, K, seed=s)).cuda() for s in (3, 4)]
     ops.set_option("pdl", -1)
-    want = [ops.gemv(fmt, W, x, N) for W, x in zip(Ws, xs)]
+    gemv = ops.gemv if M <= 8 else ops.gemm
+    want = [gemv(fmt, W, x, N) for W, x in zip(Ws, xs)]
     ops.set_option("pdl", 0)
     W, x = torch.empty_like(Ws[0]), torch.empty_like(xs[0])
 
@@ -34,7 +36,7 @@ def test_predecessor_writes_the_operands(fmt, N, K, M, ops_pdl):
     outs = []
     for i in range(12):
         load(i)
-        outs.append(ops.gemv(fmt, W, x, N))
+        outs.append(gemv(fmt, W, x, N))
     side, graph, captured = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
     torch.cuda.synchronize()
     with torch.cuda.graph(graph):
@@ -43,10 +45,10 @@ def test_predecessor_writes_the_operands(fmt, N, K, M, ops_pdl):
             load(i)
             side.wait_stream(main)
             with torch.cuda.stream(side):
-                a = ops.gemv(fmt, W, x, N)
-            b = ops.gemv(fmt, W, x, N)
+                a = gemv(fmt, W, x, N)
+            b = gemv(fmt, W, x, N)
             main.wait_stream(side)
-            captured.append((i, a, b, ops.gemv(fmt, W, x, N)))
+            captured.append((i, a, b, gemv(fmt, W, x, N)))
     for _ in range(3):
         graph.replay()
     torch.cuda.synchronize()
