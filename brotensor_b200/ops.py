@@ -14,8 +14,14 @@ from .synth import BLOCK_BYTES, BLOCK_ELEMS
 _DT = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+def _launch(t: torch.Tensor, f, *args) -> int:
+    """f(*args, stream) with t's device current; the device is switched only when it is another one (entering and leaving
+    torch.cuda.device and wrapping the stream in an object were a third of a small call's time on the host)."""
+    i = t.device.index
+    if i == torch._C._cuda_getDevice():
+        return f(*args, torch._C._cuda_getCurrentRawStream(i))
+    with torch.cuda.device(t.device):  # refuses a tensor that is not on a CUDA device
+        return f(*args, torch._C._cuda_getCurrentRawStream(i))
 
 
 def _check_w(fmt: int, W: torch.Tensor, N: int, K: int) -> None:
@@ -37,8 +43,7 @@ def repack(fmt: int, W: torch.Tensor, N: int, K: int, inplace: bool = False) -> 
     """Raw GGUF rows -> the layout the kernels read fastest (same size, bit-identical content)."""
     _check_w(fmt, W, N, K)
     out = W if inplace else torch.empty_like(W)
-    with torch.cuda.device(W.device):
-        capi.check(capi.lib().b200q_repack(fmt, W.data_ptr(), out.data_ptr(), N, K, _stream()))
+    capi.check(_launch(W, capi.lib().b200q_repack, fmt, W.data_ptr(), out.data_ptr(), N, K))
     return out
 
 
@@ -46,16 +51,14 @@ def unpack(fmt: int, W: torch.Tensor, N: int, K: int, inplace: bool = False) -> 
     """Inverse of repack; `fmt` is the raw format."""
     _check_w(fmt, W, N, K)
     out = W if inplace else torch.empty_like(W)
-    with torch.cuda.device(W.device):
-        capi.check(capi.lib().b200q_unpack(fmt, W.data_ptr(), out.data_ptr(), N, K, _stream()))
+    capi.check(_launch(W, capi.lib().b200q_unpack, fmt, W.data_ptr(), out.data_ptr(), N, K))
     return out
 
 
 def dequant(fmt: int, W: torch.Tensor, N: int, K: int, out_dtype=torch.float16) -> torch.Tensor:
     _check_w(fmt, W, N, K)
     out = torch.empty((N, K), dtype=out_dtype, device=W.device)
-    with torch.cuda.device(W.device):
-        capi.check(capi.lib().b200q_dequant(fmt, W.data_ptr(), out.data_ptr(), _DT[out_dtype], N, K, _stream()))
+    capi.check(_launch(W, capi.lib().b200q_dequant, fmt, W.data_ptr(), out.data_ptr(), _DT[out_dtype], N, K))
     return out
 
 
@@ -66,8 +69,7 @@ def embedding_gather(fmt: int, table: torch.Tensor, idx: torch.Tensor, rows: int
         raise ValueError("idx must be a contiguous CUDA int32 tensor")
     B = idx.numel()
     out = torch.empty((B, K), dtype=out_dtype, device=table.device)
-    with torch.cuda.device(table.device):
-        capi.check(capi.lib().b200q_embedding_gather(fmt, table.data_ptr(), idx.data_ptr(), B, rows, K, out.data_ptr(), _DT[out_dtype], _stream()))
+    capi.check(_launch(table, capi.lib().b200q_embedding_gather, fmt, table.data_ptr(), idx.data_ptr(), B, rows, K, out.data_ptr(), _DT[out_dtype]))
     return out
 
 
@@ -84,20 +86,19 @@ def _linear(entry: str, fmt, W, X, N, bias, out, out_dtype, ws):
         out = torch.empty((M, N), dtype=out_dtype or (torch.float16 if X.dtype == torch.float16 else torch.float32),
                           device=X.device)
     L = capi.lib()
-    bptr = bias.data_ptr() if bias is not None else None
-    with torch.cuda.device(W.device):
-        if entry in ("gemv", "gemm_static"):
-            f = L.b200q_gemv if entry == "gemv" else L.b200q_gemm_static
-            rc = f(fmt, W.data_ptr(), X.data_ptr(), _DT[X.dtype], bptr, out.data_ptr(), _DT[out.dtype],
-                              M, N, K, _stream())
-        else:
-            need = L.b200q_gemm_workspace_bytes(fmt, _DT[X.dtype], M, N, K)
-            if ws is None and need:
+    xt = _DT[X.dtype]
+    args = (fmt, W.data_ptr(), X.data_ptr(), xt, bias.data_ptr() if bias is not None else None, out.data_ptr(), _DT[out.dtype], M, N, K)
+    if entry == "gemv":
+        capi.check(_launch(W, L.b200q_gemv, *args))
+    elif entry == "gemm_static":
+        capi.check(_launch(W, L.b200q_gemm_static, *args))
+    else:
+        if ws is None and M > 8:  # decode sizes need no workspace
+            need = L.b200q_gemm_workspace_bytes(fmt, xt, M, N, K)
+            if need:
                 ws = torch.empty(need, dtype=torch.uint8, device=X.device)
-            f = L.b200q_gemm if entry == "gemm" else L.b200q_linear
-            rc = f(fmt, W.data_ptr(), X.data_ptr(), _DT[X.dtype], bptr, out.data_ptr(), _DT[out.dtype], M, N, K,
-                   ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, _stream())
-    capi.check(rc)
+        capi.check(_launch(W, L.b200q_gemm if entry == "gemm" else L.b200q_linear, *args, ws.data_ptr() if ws is not None else None,
+                           ws.numel() if ws is not None else 0))
     return out
 
 
@@ -114,9 +115,8 @@ def gemv_swiglu(fmt, W_gate, W_up, x, N, out=None, out_dtype=None):
     _check_w(fmt, W_up, N, K)
     if out is None:
         out = torch.empty((1, N), dtype=out_dtype or (torch.float16 if x.dtype == torch.float16 else torch.float32), device=x.device)
-    with torch.cuda.device(x.device):
-        capi.check(capi.lib().b200q_gemv_swiglu(fmt, W_gate.data_ptr(), W_up.data_ptr(), x.data_ptr(), _DT[x.dtype],
-                                               out.data_ptr(), _DT[out.dtype], N, K, _stream()))
+    capi.check(_launch(x, capi.lib().b200q_gemv_swiglu, fmt, W_gate.data_ptr(), W_up.data_ptr(), x.data_ptr(), _DT[x.dtype],
+                       out.data_ptr(), _DT[out.dtype], N, K))
     return out
 
 
@@ -133,9 +133,7 @@ def gemv_multi(fmt, Ws, x, Ns, outs=None, biases=None):
     Yp = (C.c_void_p * n)(*[y.data_ptr() for y in outs])
     Np = (C.c_int * n)(*Ns)
     Bp = None if biases is None else (C.c_void_p * n)(*[(b.data_ptr() if b is not None else None) for b in biases])
-    with torch.cuda.device(x.device):
-        rc = capi.lib().b200q_gemv_multi(fmt, n, Wp, Np, Yp, Bp, x.data_ptr(), _DT[x.dtype], _DT[outs[0].dtype], K, _stream())
-    capi.check(rc)
+    capi.check(_launch(x, capi.lib().b200q_gemv_multi, fmt, n, Wp, Np, Yp, Bp, x.data_ptr(), _DT[x.dtype], _DT[outs[0].dtype], K))
     return outs
 
 
@@ -153,10 +151,8 @@ def gemv_multi_rmsnorm(fmt, Ws, x, gamma, eps, Ns, outs=None):
     Wp = (C.c_void_p * n)(*[W.data_ptr() for W in Ws])
     Yp = (C.c_void_p * n)(*[y.data_ptr() for y in outs])
     Np = (C.c_int * n)(*Ns)
-    with torch.cuda.device(x.device):
-        rc = capi.lib().b200q_gemv_multi_rmsnorm(fmt, n, Wp, Np, Yp, None, x.data_ptr(), _DT[x.dtype], gamma.data_ptr(), float(eps),
-                                                 _DT[outs[0].dtype], K, _stream())
-    capi.check(rc)
+    capi.check(_launch(x, capi.lib().b200q_gemv_multi_rmsnorm, fmt, n, Wp, Np, Yp, None, x.data_ptr(), _DT[x.dtype], gamma.data_ptr(), float(eps),
+                       _DT[outs[0].dtype], K))
     return outs
 
 
