@@ -38,18 +38,13 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict_
 // Eight values, rounded once to the output type, to consecutive positions.
 template <typename OT>
 __device__ __forceinline__ void dq_store8(OT* o, const float (&f)[8]) {
-    if constexpr (sizeof(OT) == 4) {
-        reinterpret_cast<float4*>(o)[0] = make_float4(f[0], f[1], f[2], f[3]);
-        reinterpret_cast<float4*>(o)[1] = make_float4(f[4], f[5], f[6], f[7]);
-    } else {
-        union {
-            OT h[8];
-            uint4 v;
-        } pk;
+    union {
+        OT h[8];
+        uint4 v;
+    } pk;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) pk.h[k] = from_f32<OT>(f[k]);
-        *reinterpret_cast<uint4*>(o) = pk.v;
-    }
+    for (int k = 0; k < 8; ++k) pk.h[k] = from_f32<OT>(f[k]);
+    *reinterpret_cast<uint4*>(o) = pk.v;
 }
 
 // Q4_K and Q5_K, one thread per eight positions of two neighbouring 64-element groups: the block header (one
@@ -157,6 +152,60 @@ __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* W, OT* 
     }
 }
 
+// Q8_0 and Q4_0, 32 values per thread as well: of Q8_0 eight consecutive ones in each of four neighbouring blocks, of Q4_0 eight
+// bytes - a half block's low nibbles and the high ones sixteen positions on - in each of two. Blocks are 34 and 18 bytes, so every
+// other one has its quants on a word boundary and the ones between two bytes behind one (a funnel shift). Needs rows of whole
+// groups (K a multiple of 128 / 64) on a 4-byte boundary. d * q is exact in FP32, one rounding to the output type.
+__device__ __forceinline__ uint32_t ld_dep_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+template <int FMT, typename OT>
+__global__ void __launch_bounds__(256) dequant_32_kernel(const uint8_t* W, OT* out, long long total_units, int units_per_row, int row_bytes, int K) {
+    constexpr int kBlock = FMT == kQ8_0 ? 34 : 18, kBlocks = FMT == kQ8_0 ? 4 : 2, kParts = FMT == kQ8_0 ? 4 : 2;
+    grid_dep_launch();
+    grid_dep_wait();
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < total_units; id += stride) {
+        const long long r = id / units_per_row;
+        const int u = (int)(id - r * units_per_row), group = u / kParts, p = u % kParts;
+        const uint8_t* g = W + (size_t)r * row_bytes + (size_t)group * (kBlocks * kBlock);
+        uint32_t q[kBlocks][2];
+        float d[kBlocks];
+#pragma unroll
+        for (int j = 0; j < kBlocks; ++j) {
+            const uint8_t* b = g + kBlock * j + 8 * p;
+            d[j] = h2f(ld_dep_u16(g + kBlock * j));
+            if (j & 1) {
+                q[j][0] = ld_dep_u32(b + 2);
+                q[j][1] = ld_dep_u32(b + 6);
+            } else {
+                const uint32_t w0 = ld_dep_u32(b), w1 = ld_dep_u32(b + 4), w2 = ld_dep_u32(b + 8);
+                q[j][0] = __funnelshift_r(w0, w1, 16);
+                q[j][1] = __funnelshift_r(w1, w2, 16);
+            }
+        }
+        OT* o = out + (size_t)r * K + (size_t)group * (32 * kBlocks) + 8 * p;
+#pragma unroll
+        for (int j = 0; j < kBlocks; ++j) {
+#pragma unroll
+            for (int h = 0; h < (FMT == kQ8_0 ? 1 : 2); ++h) {
+                float f[8];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    // byte + 128 / nibble, as 2^23 + value
+                    const uint32_t v = FMT == kQ8_0 ? q[j][k] ^ 0x80808080u : (q[j][k] >> (4 * h)) & 0x0F0F0F0Fu;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        f[4 * k + i] = d[j] * (__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 | i)) - (FMT == kQ8_0 ? 8388736.0f : 8388616.0f));
+                }
+                dq_store8<OT>(o + 32 * j + 16 * h, f);
+            }
+        }
+    }
+}
+
 // The wide kernels' launch: 32 values per thread.
 template <typename OT>
 static int launch_dequant_wide(void (*kern)(const uint8_t*, OT*, long long, int, int, int), const uint8_t* W, void* out, int64_t rows, int K, int row_bytes,
@@ -170,6 +219,7 @@ static int launch_dequant_wide(void (*kern)(const uint8_t*, OT*, long long, int,
 template <int FMT, typename OT>
 static int launch_dequant_wide_f(const uint8_t* W, void* out, int64_t rows, int K, int row_bytes, long long cap, cudaStream_t st) {
     if constexpr (FMT == kQ4_K || FMT == kQ5_K) return launch_dequant_wide<OT>(dequant_k_kernel<FMT, OT>, W, out, rows, K, row_bytes, cap, st);
+    else if constexpr (FMT == kQ8_0 || FMT == kQ4_0) return launch_dequant_wide<OT>(dequant_32_kernel<FMT, OT>, W, out, rows, K, row_bytes, cap, st);
     else return launch_dequant_wide<OT>(dequant_q6k_kernel<FMT == kQ6_KP, OT>, W, out, rows, K, row_bytes, cap, st);
 }
 
@@ -182,14 +232,16 @@ static int launch_dequant_fmt(const void* W, void* out, int out_dtype, int64_t r
     const long long cap = 148LL * 8 * 16;
     if (blocks > cap) blocks = cap;
     const uint8_t* w = static_cast<const uint8_t*>(W);
-    if constexpr (FMT == kQ4_K || FMT == kQ5_K || FMT == kQ6_K || FMT == kQ6_KP) {
-        // (the K-quant kernels load whole headers; Q6_K takes any block address)
-        if (FMT == kQ6_K || FMT == kQ6_KP || (reinterpret_cast<uintptr_t>(W) & 15) == 0) {
-            switch (out_dtype) {
-                case B200Q_DT_F16: return launch_dequant_wide_f<FMT, __half>(w, out, rows, K, row_bytes, cap, st);
-                case B200Q_DT_BF16: return launch_dequant_wide_f<FMT, __nv_bfloat16>(w, out, rows, K, row_bytes, cap, st);
-                case B200Q_DT_F32: return launch_dequant_wide_f<FMT, float>(w, out, rows, K, row_bytes, cap, st);
-            }
+    if (out_dtype == B200Q_DT_F16 || out_dtype == B200Q_DT_BF16) {
+        // The wide kernels: 16-bit outputs. With FP32 a thread's 32-byte pieces lie apart and every store instruction of a warp leaves
+        // half sectors; seven matrices of a 4096 / 14336 layer, wide against generic, us: FP16 Q8_0 134 / 163, Q4_0 110 / 165, BF16 Q4_K
+        // and Q6_K 104 / 183, but FP32 Q8_0 242 / 223, Q4_0 342 / 212, Q4_K and Q6_K 240 / 234.
+        // Q4_K and Q5_K load whole headers, Q8_0 and Q4_0 words of groups of blocks; Q6_K takes any block address.
+        const uintptr_t at = reinterpret_cast<uintptr_t>(W);
+        if (FMT == kQ6_K || FMT == kQ6_KP || ((FMT == kQ4_K || FMT == kQ5_K) && (at & 15) == 0) ||
+            (FMT == kQ8_0 && K % 128 == 0 && (at & 3) == 0) || (FMT == kQ4_0 && K % 64 == 0 && (at & 3) == 0)) {
+            if (out_dtype == B200Q_DT_F16) return launch_dequant_wide_f<FMT, __half>(w, out, rows, K, row_bytes, cap, st);
+            return launch_dequant_wide_f<FMT, __nv_bfloat16>(w, out, rows, K, row_bytes, cap, st);
         }
     }
     switch (out_dtype) {

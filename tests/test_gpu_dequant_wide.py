@@ -1,5 +1,5 @@
-"""The K-quant decode kernels (32 values per thread) in every output type, bit for bit against the oracle: rows of one block and of an odd number
-of blocks, sizes below and above one thread block, the regrouped Q6_K layout, and weights that are not aligned for whole-header
+"""The wide decode kernels (32 values per thread, 16-bit outputs) and the generic one behind FP32, bit for bit against the oracle: rows of one
+block and of an odd number of blocks, sizes below and above one thread block, the regrouped Q6_K layout, and weights that are not aligned for whole-header
 loads (those take the generic kernel)."""
 import numpy as np
 import pytest
@@ -38,3 +38,15 @@ def test_decode_is_exact(fmt, rows, K):
         if fmt == synth.Q6_K and K % 2048 == 0:
             R = ops.repack(fmt, W, rows, K)
             assert np.array_equal(_bits(ops.dequant(ops.repacked_fmt(fmt, K), R, rows, K, dt), dt), want.reshape(rows, K))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,K", [(1, 32), (7, 96), (5, 64), (33, 320), (9, 384)])
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0])
+def test_rows_of_a_few_blocks(fmt, rows, K):
+    """Rows that are not whole groups of four (Q8_0) or two (Q4_0) blocks take the generic kernel."""
+    from brotensor_b200 import ops
+    Wh = synth.make_blocks(fmt, rows, K, seed=rows + K)
+    W = torch.from_numpy(Wh).cuda()
+    for dt in DT:
+        assert np.array_equal(_bits(ops.dequant(fmt, W, rows, K, dt), dt), _want(fmt, Wh, rows, K, dt).reshape(rows, K))
