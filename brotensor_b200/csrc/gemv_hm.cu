@@ -17,7 +17,8 @@
 // neighbouring 256-element blocks of the rows (and of X) as there are warps per tile, each warp multiplies one of them, and the tile's
 // warps add up at the end of the rows in a fixed order. So every warp has eight k-steps of independent work between two CTA
 // barriers however few rows there are (with stages of one block, shared by sub-blocks, 4096 x 14336 took 33 us instead of 17.6). Stages
-// are fetched with cp.async up to five ahead.
+// are fetched with cp.async up to five ahead. Where the rows take many steps and the activations are short they are kept in shared memory
+// whole, every warp has a ring of its own and no barrier is left in the loop.
 // Results that are not finite are computed again in plain FP32 (qm_plain_rows): 0 * inf on a masked quant is not what the
 // dequantised weight gives.
 //
@@ -30,6 +31,7 @@ namespace b200q {
 constexpr int kHmMaxWarps = 16;
 constexpr int kHmMaxTiles = 8;  // 16-row tiles of a CTA at a time
 constexpr int kHmMaxStages = 6;
+constexpr int kHmResident = 32768;  // activations (M * K) that are kept in shared memory for the whole launch
 
 struct HmParams {
     const uint8_t* W;
@@ -164,7 +166,9 @@ __device__ __forceinline__ void hm_scales(const QmRow& r, float d, uint32_t sc_l
     }
 }
 
-template <int FMT, bool BF>
+// XRES: the activations are short enough to lie in shared memory whole (M * K <= kHmResident). Then a warp needs nothing but its own copies
+// and the warps run without a barrier until the rows are done.
+template <int FMT, bool BF, bool XRES>
 __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __grid_constant__ HmParams p) {
     using F = QmFmt<FMT>;
     extern __shared__ uint8_t smem_raw[];
@@ -182,7 +186,10 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
     // A warp copies what it multiplies - rows g and g + 8 of its tile, four threads each, of its block - and the first tile's warps
     // the activations of their block, a row of X per instruction. The 16-byte chunks of X are rotated so that the threads that read
     // together - 16 bytes each from two rows, or 8 bytes each from four - find them in different banks.
-    const uint32_t my_rows = (uint32_t)(((ki * p.mt + mi) * kQmTile + g) * F::stride), my_x = (uint32_t)p.off_x + (uint32_t)(ki * p.M * 512);
+    constexpr uint32_t kTileBytes = kQmTile * F::stride;
+    // a slot's bytes of this lane's row g: with XRES in the warp's own ring, else in the CTA's
+    const uint32_t slot_bytes = XRES ? kTileBytes : (uint32_t)p.stage_bytes;
+    const uint32_t my_rows = (XRES ? (uint32_t)(warp * p.n_stages) : (uint32_t)(ki * p.mt + mi)) * kTileBytes + (uint32_t)(g * F::stride), my_x = (uint32_t)p.off_x + (uint32_t)(ki * p.M * 512);
     const size_t row8 = (size_t)8 * p.row_bytes, k_step = (size_t)p.kg * F::bytes, it_step = (size_t)rows_it * p.row_bytes;
     const uint8_t* const src0 = p.W + (size_t)(row_begin + mi * kQmTile + g) * p.row_bytes + (size_t)ki * F::bytes;
     const uint8_t* const x0 = p.X + 512 * (size_t)ki + 16 * lane;
@@ -191,11 +198,11 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
     auto issue = [&] {
         if (ii < iters) {
             if (is * p.kg + ki < p.nblk) {
-                const uint32_t st = sbase + (uint32_t)(islot * p.stage_bytes);
+                const uint32_t st = sbase + (uint32_t)islot * slot_bytes;
                 const int r = ii * rows_it + mi * kQmTile + g;
                 if (r < n_rows) qm_copy_row<FMT>(st + my_rows, isrc, t);
                 if (r + 8 < n_rows) qm_copy_row<FMT>(st + my_rows + 8u * F::stride, isrc + row8, t);
-                if (mi == 0) {
+                if (!XRES && mi == 0) {
                     const uint8_t* x = xsrc;
                     for (int m = 0; m < p.M; ++m, x += 2 * (size_t)p.K) {
                         const uint32_t sw = F::pair8 ? (uint32_t)(m & 1) << 2 : (uint32_t)(m & 3) << 1;
@@ -222,6 +229,16 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
     }
     grid_dep_wait();
     for (int s = 0; s < p.n_stages - 1; ++s) issue();
+    if constexpr (XRES) {
+        for (int i = warp; i < p.nblk * p.M; i += p.mt * p.kg) {  // row m of block b
+            const int b = i / p.M, m = i - b * p.M;
+            const uint32_t sw = F::pair8 ? (uint32_t)(m & 1) << 2 : (uint32_t)(m & 3) << 1;
+            cp_async16(sbase + (uint32_t)p.off_x + (uint32_t)(i * 512) + (((uint32_t)lane ^ sw) << 4), p.X + ((size_t)m * p.K + 256 * (size_t)b) * 2 + 16 * lane);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+    }
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     int slot = 0, it = 0, ks = 0;
@@ -234,11 +251,13 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
             case 3: cp_async_wait<1>(); break;
             default: cp_async_wait<0>(); break;
         }
-        __syncthreads();  // the stage has landed for everybody, and everybody is done with the slot filled next
+        // the stage has landed for everybody who reads it, and everybody is done with the slot filled next
+        if constexpr (XRES) __syncwarp();
+        else __syncthreads();
         issue();
         const int r0 = it * rows_it + mi * kQmTile;
         if (r0 < n_rows && ks * p.kg + ki < p.nblk) {
-            const uint8_t* st = smem + slot * p.stage_bytes;
+            const uint8_t* st = smem + slot * slot_bytes;
             const QmRow ra = qm_row<FMT>(st + my_rows, rsrc), rb = qm_row<FMT>(st + my_rows + 8 * F::stride, rsrc + row8);
             float dA = 0.f, dB = 0.f, mA = 0.f, mB = 0.f;
             uint32_t sc[2][2] = {{0, 0}, {0, 0}}, mn[2][2] = {{0, 0}, {0, 0}};
@@ -252,7 +271,7 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
                 dA = h2f((ls32(ra.p + 208) >> ra.sh) & 0xFFFFu);
                 dB = h2f((ls32(rb.p + 208) >> rb.sh) & 0xFFFFu);
             }
-            const uint8_t* xrow = st + my_x + g * 512;
+            const uint8_t* xrow = XRES ? smem + p.off_x + ((ks * p.kg + ki) * p.M + g) * 512 : st + my_x + g * 512;
             float cm[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
@@ -313,7 +332,8 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
         // ---- these rows are done: add up the tile's warps (in order), store
         ks = 0;
         if (p.kg > 1) {
-            const uint32_t red = sbase + (uint32_t)p.off_red + (uint32_t)(lane * 16);
+            // (two buffers in turn where no stage barrier keeps the next rows' sums from overtaking the reads of these)
+            const uint32_t red = sbase + (uint32_t)p.off_red + (uint32_t)(lane * 16) + (XRES && (it & 1) ? (uint32_t)((p.kg - 1) * p.mt * 512) : 0u);
             if (ki > 0)
                 sts128(red + (uint32_t)(((ki - 1) * p.mt + mi) * 512),
                        make_uint4(__float_as_uint(acc[0]), __float_as_uint(acc[1]), __float_as_uint(acc[2]), __float_as_uint(acc[3])));
@@ -358,9 +378,9 @@ static int g_opt_hm = 1;
 void hm_set_enabled(int v) { g_opt_hm = v < 0 ? 0 : (v > 2 ? 2 : v); }
 int hm_get_enabled() { return g_opt_hm; }
 
-template <int FMT, bool BF>
+template <int FMT, bool BF, bool XRES>
 static int launch_hm(const HmParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = gemv_hm_kernel<FMT, BF>;
+    auto kern = gemv_hm_kernel<FMT, BF, XRES>;
     static bool configured[64] = {};
     int dev = 0;
     B200Q_CUDA_TRY(cudaGetDevice(&dev));
@@ -387,6 +407,21 @@ static int launch_hm_f(HmParams& p, bool bf, int sms, cudaStream_t st, bool* tak
     int kg = kHmMaxWarps / p.mt;
     p.k_stages = (p.nblk + kg - 1) / kg;
     p.kg = kg = (p.nblk + p.k_stages - 1) / p.k_stages;
+    // Activations resident, no stage barrier: 14336 x 4096 Q4_K (8 steps) 18.9 -> 17.2 us, 32000 x 4096 (16) 37.5 -> 31.5, 4096 x 14336 one row (7)
+    // 17.5 -> 16.9; but the start waits for all of X, so short runs lose: 4096 x 4096 (2 steps) 6.5 -> 7.2, 2560 x 6912 (4) 8.8 -> 9.3.
+    if ((long long)p.M * p.K <= kHmResident && iters * p.k_stages >= 6) {
+        const size_t x = (size_t)p.nblk * p.M * 512, red = 2 * (size_t)(kg - 1) * p.mt * 512, tail = red > 3584 ? red : 3584, budget = 227 * 1024 - 1024 - 256;
+        const size_t tile = (size_t)p.mt * kg * kQmTile * F::stride;
+        p.n_stages = kHmMaxStages;
+        while (p.n_stages > 2 && p.n_stages * tile + x + tail > budget) --p.n_stages;
+        if (p.n_stages * tile + x + tail <= budget) {
+            p.off_x = (int)(p.n_stages * tile);
+            p.off_red = p.off_x + (int)x;
+            *taken = true;
+            const size_t smem = (size_t)p.off_red + tail + 128;
+            return bf ? launch_hm<FMT, true, true>(p, grid, smem, st) : launch_hm<FMT, false, true>(p, grid, smem, st);
+        }
+    }
     p.off_x = p.mt * kg * kQmTile * F::stride;
     p.stage_bytes = (p.off_x + kg * p.M * 512 + 127) & ~127;
     // (rows past M of the last block's activations are read, not used: up to 7 x 512 bytes past the stage)
@@ -398,7 +433,7 @@ static int launch_hm_f(HmParams& p, bool bf, int sms, cudaStream_t st, bool* tak
     p.off_red = p.n_stages * p.stage_bytes;
     *taken = true;
     const size_t smem = (size_t)p.off_red + tail + 128;
-    return bf ? launch_hm<FMT, true>(p, grid, smem, st) : launch_hm<FMT, false>(p, grid, smem, st);
+    return bf ? launch_hm<FMT, true, false>(p, grid, smem, st) : launch_hm<FMT, false, false>(p, grid, smem, st);
 }
 
 // Launches the kernel when it takes the call (*taken = true): FP16 or BF16 activations, K a multiple of 256, weights on a 16-byte boundary

@@ -35,7 +35,7 @@ def _operands(fmt, N, K, M, dtype):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,K", SHAPES)
+@pytest.mark.parametrize("N,K", SHAPES + [(40000, 768)])  # the last: several row sets per CTA, activations resident in gemv_hm
 @pytest.mark.parametrize("fmt", FMTS)
 def test_decode_rows(fmt, N, K, ops_raw):
     ops = ops_raw
