@@ -15,7 +15,7 @@ LIB_PATH = os.environ.get("B200Q_LIB") or os.path.join(PKG, "lib", "libb200q.so"
 OK = 0
 ERR_BAD_ARG, ERR_UNSUPPORTED, ERR_CUDA, ERR_TIMEOUT, ERR_WORKSPACE = 1, 2, 3, 4, 5
 Q8_0, Q4_K, Q6_K = 14, 22, 24
-Q4_0, Q5_K = 10, 23  # carried by brotensor's loader without ops; decode, GEMV (plain-load kernel) and gather here
+Q4_0, Q5_K = 10, 23  # carried by brotensor's loader without ops; decode, GEMV, GEMM and gather here
 Q6_K_R8 = 124  # Q6_K regrouped by field in runs of eight blocks (b200q_repack)
 F32, F16, BF16 = 0, 1, 4
 

@@ -132,7 +132,7 @@ static bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 // Alignment a weight pointer needs for its block header loads.
 static size_t w_align(int fmt) { return fmt == kQ6_KP ? 16 : (fmt == kQ4_K || fmt == kQ5_K) ? 4 : 2; }
 // Formats the streaming decode kernels, the tensor-core GEMM and the fused / sharded forms take; the
-// others (Q4_0, Q5_K) run through the plain-load GEMV.
+// others (Q4_0, Q5_K) have the raw-quant kernels and the plain-load GEMV.
 static bool streaming_fmt(int fmt) { return fmt == kQ4_K || fmt == kQ6_K || fmt == kQ6_KP || fmt == kQ8_0; }
 
 static int check_linear_args(const char* op, int fmt, const void* W, const void* X, int x_dtype, const void* Y,

@@ -284,7 +284,8 @@ int b200q_device_status(int* status_out);
  *                 one pipeline with 32-row tiles; "gemv_split_full" (Q6_K only) -1 = automatic, 0 = one full
  *                 barrier per stage, 1 = one per consumer warp and stage
  *   "gemm_path"   0 = automatic (tcgen05 GEMM from 9 rows, except 9..16 rows of Q4_K / Q8_0 with K = 2048 / 4096 and
- *                 of Q6_K from 8192 weight rows, which run as two passes of the small-batch GEMV), 1 = passes of the
+ *                 of Q6_K from 8192 weight rows, and of matrices up to 8192 rows with 16-bit activations, which run as
+ *                 two passes of the small-batch GEMV; Q5_K and Q4_0: "gemm_mm"), 1 = passes of the
  *                 decode GEMV only, 2 = the tcgen05 GEMM or an error
  *   "gemm_pair"   0 = one-CTA tcgen05 kernel, otherwise the CTA-pair kernel (default)
  *   "gemm_split"  0 = never split K; 1 (default) = where it shortens the call, matrices of few row tiles
