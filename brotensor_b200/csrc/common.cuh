@@ -133,6 +133,49 @@ __device__ __forceinline__ uint32_t ld_w(const uint8_t* p) {
     if constexpr (ALIGN >= 4) return ld_nc_u32(p);
     else return ld_nc_u32_a2(p);
 }
+// Loads of what the stream's predecessor may have written, for kernels that start before it has finished: ordinary
+// coherent loads that stay behind griddepcontrol.wait (the read-only path promises data that nobody
+// writes while the kernel lives, and its loads may be moved).
+__device__ __forceinline__ uint4 ld_dep_u4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_dep_u16(const void* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_dep_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_dep_u2(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_dep_f4(const void* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+// The two sets of loads, for decode8: kernels that start behind their predecessor may use the read-only path; those that start
+// before it has finished (launch_dep) may not.
+struct LdNc {
+    static __device__ __forceinline__ uint32_t u16(const void* p) { return ld_nc_u16(p); }
+    static __device__ __forceinline__ uint32_t u32(const void* p) { return ld_nc_u32(p); }
+    static __device__ __forceinline__ uint2 u2(const void* p) { return __ldg(reinterpret_cast<const uint2*>(p)); }
+};
+struct LdDep {
+    static __device__ __forceinline__ uint32_t u16(const void* p) { return ld_dep_u16(p); }
+    static __device__ __forceinline__ uint32_t u32(const void* p) { return ld_dep_u32(p); }
+    static __device__ __forceinline__ uint2 u2(const void* p) { return ld_dep_u2(p); }
+};
+// 4 bytes from an address that is only 2-byte aligned.
+template <class LD>
+__device__ __forceinline__ uint32_t ld_u32_a2(const uint8_t* p) { return LD::u16(p) | (LD::u16(p + 2) << 16); }
 __device__ __forceinline__ float h2f(uint32_t bits16) { return __half2float(__ushort_as_half((unsigned short)bits16)); }
 
 // ---- exact decode of 8 consecutive elements -----------------------------------
@@ -140,15 +183,12 @@ __device__ __forceinline__ float h2f(uint32_t bits16) { return __half2float(__us
 // consecutive elements along the row. Every product below is exact in FP32 and
 // the single subtraction rounds the exact value, so the result is independent of
 // operation order and FMA contraction.
-template <int FMT>
-__device__ __forceinline__ void decode8(const uint8_t* __restrict__ row, int u, float w[8]);
-
-template <>
-__device__ __forceinline__ void decode8<kQ4_K>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q4k(const uint8_t* row, int u, float w[8]) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 144;
     const int i = u & 31, is = i >> 2, l0 = (i & 3) * 8;
-    const uint32_t dd = ld_nc_u32(blk);
-    const uint32_t s0 = ld_nc_u32(blk + 4), s1 = ld_nc_u32(blk + 8), s2 = ld_nc_u32(blk + 12);
+    const uint32_t dd = LD::u32(blk);
+    const uint32_t s0 = LD::u32(blk + 4), s1 = LD::u32(blk + 8), s2 = LD::u32(blk + 12);
     uint32_t sc, m;
     if (is < 4) {
         sc = (s0 >> (8 * is)) & 63u;
@@ -161,7 +201,7 @@ __device__ __forceinline__ void decode8<kQ4_K>(const uint8_t* __restrict__ row, 
     const float ds = h2f(dd & 0xFFFFu) * (float)sc;
     const float dm = h2f(dd >> 16) * (float)m;
     const uint8_t* q = blk + 16 + (is >> 1) * 32 + l0;
-    uint32_t q0 = ld_nc_u32(q), q1 = ld_nc_u32(q + 4);
+    uint32_t q0 = LD::u32(q), q1 = LD::u32(q + 4);
     if (is & 1) {
         q0 >>= 4;
         q1 >>= 4;
@@ -173,22 +213,22 @@ __device__ __forceinline__ void decode8<kQ4_K>(const uint8_t* __restrict__ row, 
     }
 }
 
-template <>
-__device__ __forceinline__ void decode8<kQ6_K>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q6k(const uint8_t* row, int u, float w[8]) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 210;
     const int i = u & 31, group = i >> 4, quad = (i & 15) >> 2, l0 = (i & 3) * 8;
     const int sb = group * 8 + quad * 2 + (l0 >> 4);
     const uint8_t* ql = blk + group * 64 + (quad & 1) * 32 + l0;
     const uint8_t* qh = blk + 128 + group * 32 + l0;
-    uint32_t a0 = ld_nc_u32_a2(ql), a1 = ld_nc_u32_a2(ql + 4);
-    const uint32_t h0 = ld_nc_u32_a2(qh) >> (quad * 2), h1 = ld_nc_u32_a2(qh + 4) >> (quad * 2);
+    uint32_t a0 = ld_u32_a2<LD>(ql), a1 = ld_u32_a2<LD>(ql + 4);
+    const uint32_t h0 = ld_u32_a2<LD>(qh) >> (quad * 2), h1 = ld_u32_a2<LD>(qh + 4) >> (quad * 2);
     if (quad >= 2) {
         a0 >>= 4;
         a1 >>= 4;
     }
-    const uint32_t scd = ld_nc_u16(blk + 192 + (sb & ~1));
+    const uint32_t scd = LD::u16(blk + 192 + (sb & ~1));
     const int sc = (int)(signed char)((scd >> ((sb & 1) * 8)) & 0xFFu);
-    const float ds = h2f(ld_nc_u16(blk + 208)) * (float)sc;
+    const float ds = h2f(LD::u16(blk + 208)) * (float)sc;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int v0 = (int)(((a0 >> (8 * k)) & 0xFu) | (((h0 >> (8 * k)) & 3u) << 4)) - 32;
@@ -198,23 +238,23 @@ __device__ __forceinline__ void decode8<kQ6_K>(const uint8_t* __restrict__ row, 
     }
 }
 
-template <>
-__device__ __forceinline__ void decode8<kQ6_KP>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q6kp(const uint8_t* row, int u, float w[8]) {
     const int b = u >> 5;  // block along the row; run b >> 3, slot b & 7
     const uint8_t* run = row + (size_t)(b >> 3) * kQ6RunBytes;
     const int s = b & 7;
     const int i = u & 31, group = i >> 4, quad = (i & 15) >> 2, l0 = (i & 3) * 8;
     const int sb = group * 8 + quad * 2 + (l0 >> 4);
-    const uint2 a = __ldg(reinterpret_cast<const uint2*>(run + s * 128 + group * 64 + (quad & 1) * 32 + l0));
-    const uint2 h = __ldg(reinterpret_cast<const uint2*>(run + 1024 + s * 64 + group * 32 + l0));
+    const uint2 a = LD::u2(run + s * 128 + group * 64 + (quad & 1) * 32 + l0);
+    const uint2 h = LD::u2(run + 1024 + s * 64 + group * 32 + l0);
     uint32_t a0 = a.x, a1 = a.y;
     const uint32_t h0 = h.x >> (quad * 2), h1 = h.y >> (quad * 2);
     if (quad >= 2) {
         a0 >>= 4;
         a1 >>= 4;
     }
-    const int sc = (int)(signed char)__ldg(run + 1536 + s * 16 + sb);
-    const float ds = h2f(ld_nc_u16(run + 1664 + 2 * s)) * (float)sc;
+    const int sc = (int)(signed char)(LD::u16(run + 1536 + s * 16 + (sb & ~1)) >> ((sb & 1) * 8) & 0xFFu);
+    const float ds = h2f(LD::u16(run + 1664 + 2 * s)) * (float)sc;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int v0 = (int)(((a0 >> (8 * k)) & 0xFu) | (((h0 >> (8 * k)) & 3u) << 4)) - 32;
@@ -224,12 +264,12 @@ __device__ __forceinline__ void decode8<kQ6_KP>(const uint8_t* __restrict__ row,
     }
 }
 
-template <>
-__device__ __forceinline__ void decode8<kQ8_0>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q8_0(const uint8_t* row, int u, float w[8]) {
     const uint8_t* blk = row + (size_t)(u >> 2) * 34;
-    const float d = h2f(ld_nc_u16(blk));
+    const float d = h2f(LD::u16(blk));
     const uint8_t* q = blk + 2 + (u & 3) * 8;
-    const uint32_t q0 = ld_nc_u32_a2(q), q1 = ld_nc_u32_a2(q + 4);
+    const uint32_t q0 = ld_u32_a2<LD>(q), q1 = ld_u32_a2<LD>(q + 4);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         w[k] = d * (float)(int)(signed char)((q0 >> (8 * k)) & 0xFFu);
@@ -239,13 +279,13 @@ __device__ __forceinline__ void decode8<kQ8_0>(const uint8_t* __restrict__ row, 
 
 // Q4_0 (ggml block_q4_0, dequantize_row_q4_0): element j of a block is the low nibble of qs[j] for
 // j < 16 and the high nibble of qs[j - 16] otherwise, minus 8, times d. d * (q - 8): 11 + 4 bits, exact.
-template <>
-__device__ __forceinline__ void decode8<kQ4_0>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q4_0(const uint8_t* row, int u, float w[8]) {
     const uint8_t* blk = row + (size_t)(u >> 2) * 18;
-    const float d = h2f(ld_nc_u16(blk));
+    const float d = h2f(LD::u16(blk));
     const int part = u & 3;  // elements 8 * part .. 8 * part + 7
     const uint8_t* q = blk + 2 + (part & 1) * 8;
-    uint32_t q0 = ld_nc_u32_a2(q), q1 = ld_nc_u32_a2(q + 4);
+    uint32_t q0 = ld_u32_a2<LD>(q), q1 = ld_u32_a2<LD>(q + 4);
     if (part >= 2) {
         q0 >>= 4;
         q1 >>= 4;
@@ -261,12 +301,12 @@ __device__ __forceinline__ void decode8<kQ4_0>(const uint8_t* __restrict__ row, 
 // qs[128] @48. Sub-block is = 0..7 of 32 elements: byte qs[(is >> 1) * 32 + l], low nibble for even is,
 // high nibble for odd; the fifth bit is bit `is` of qh[l]. w = d * sc * q - dmin * m with q in 0..31:
 // 11 + 6 + 5 bits and 11 + 6 bits, both exact in FP32, one rounding in the subtraction.
-template <>
-__device__ __forceinline__ void decode8<kQ5_K>(const uint8_t* __restrict__ row, int u, float w[8]) {
+template <class LD>
+__device__ __forceinline__ void decode8_q5k(const uint8_t* row, int u, float w[8]) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 176;
     const int i = u & 31, is = i >> 2, l0 = (i & 3) * 8;
-    const uint32_t dd = ld_nc_u32(blk);
-    const uint32_t s0 = ld_nc_u32(blk + 4), s1 = ld_nc_u32(blk + 8), s2 = ld_nc_u32(blk + 12);
+    const uint32_t dd = LD::u32(blk);
+    const uint32_t s0 = LD::u32(blk + 4), s1 = LD::u32(blk + 8), s2 = LD::u32(blk + 12);
     uint32_t sc, m;
     if (is < 4) {
         sc = (s0 >> (8 * is)) & 63u;
@@ -280,8 +320,8 @@ __device__ __forceinline__ void decode8<kQ5_K>(const uint8_t* __restrict__ row, 
     const float dm = h2f(dd >> 16) * (float)m;
     const uint8_t* q = blk + 48 + (is >> 1) * 32 + l0;
     const uint8_t* h = blk + 16 + l0;
-    uint32_t q0 = ld_nc_u32(q), q1 = ld_nc_u32(q + 4);
-    const uint32_t h0 = ld_nc_u32(h) >> is, h1 = ld_nc_u32(h + 4) >> is;
+    uint32_t q0 = LD::u32(q), q1 = LD::u32(q + 4);
+    const uint32_t h0 = LD::u32(h) >> is, h1 = LD::u32(h + 4) >> is;
     if (is & 1) {
         q0 >>= 4;
         q1 >>= 4;
@@ -291,6 +331,16 @@ __device__ __forceinline__ void decode8<kQ5_K>(const uint8_t* __restrict__ row, 
         w[k] = ds * (float)(((q0 >> (8 * k)) & 0xFu) | (((h0 >> (8 * k)) & 1u) << 4)) - dm;
         w[4 + k] = ds * (float)(((q1 >> (8 * k)) & 0xFu) | (((h1 >> (8 * k)) & 1u) << 4)) - dm;
     }
+}
+
+template <int FMT, class LD = LdNc>
+__device__ __forceinline__ void decode8(const uint8_t* row, int u, float w[8]) {
+    if constexpr (FMT == kQ4_K) decode8_q4k<LD>(row, u, w);
+    else if constexpr (FMT == kQ5_K) decode8_q5k<LD>(row, u, w);
+    else if constexpr (FMT == kQ6_K) decode8_q6k<LD>(row, u, w);
+    else if constexpr (FMT == kQ6_KP) decode8_q6kp<LD>(row, u, w);
+    else if constexpr (FMT == kQ8_0) decode8_q8_0<LD>(row, u, w);
+    else decode8_q4_0<LD>(row, u, w);
 }
 
 // ---- element type helpers -----------------------------------------------------
@@ -372,29 +422,6 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void prefetch_l2_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-// Loads of what the stream's predecessor may have written, for kernels that start before it has finished: ordinary
-// coherent loads that stay behind griddepcontrol.wait (the read-only path promises data that nobody
-// writes while the kernel lives, and its loads may be moved).
-__device__ __forceinline__ uint4 ld_dep_u4(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint32_t ld_dep_u16(const void* p) {
-    unsigned short v;
-    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint2 ld_dep_u2(const void* p) {
-    uint2 v;
-    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float4 ld_dep_f4(const void* p) {
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- warp-level MMA (FP16 operands, FP32 accumulators) ------------------------

@@ -99,7 +99,6 @@ __global__ void __launch_bounds__(256) dequant_k_kernel(const uint8_t* W, OT* ou
 // each of the half's four 32-element quarters - so four runs of stores, and the loads and the scale
 // work of the generic path are shared by four times as many outputs. Blocks are 2-byte aligned only;
 // all loads are 16-bit pairs. d * sc * (q - 32) is exact in FP32 (11 + 7 + 6 bits), one rounding to the output type.
-__device__ __forceinline__ uint32_t ld_dep_u32_a2(const uint8_t* p) { return ld_dep_u16(p) | (ld_dep_u16(p + 2) << 16); }
 template <bool RUNS, typename OT>  // RUNS: the layout regrouped by field in runs of eight blocks (16-byte aligned fields)
 __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* W, OT* out, long long total_units, int units_per_row, int row_bytes, int K) {
     grid_dep_launch();
@@ -127,9 +126,9 @@ __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* W, OT* 
             const uint8_t* blk = W + (size_t)r * row_bytes + (size_t)b * 210;
             const uint8_t* ql = blk + n * 64 + l0;
             const uint8_t* qh = blk + 128 + n * 32 + l0;
-            a[0][0] = ld_dep_u32_a2(ql); a[0][1] = ld_dep_u32_a2(ql + 4);
-            a[1][0] = ld_dep_u32_a2(ql + 32); a[1][1] = ld_dep_u32_a2(ql + 36);
-            h[0] = ld_dep_u32_a2(qh); h[1] = ld_dep_u32_a2(qh + 4);
+            a[0][0] = ld_u32_a2<LdDep>(ql); a[0][1] = ld_u32_a2<LdDep>(ql + 4);
+            a[1][0] = ld_u32_a2<LdDep>(ql + 32); a[1][1] = ld_u32_a2<LdDep>(ql + 36);
+            h[0] = ld_u32_a2<LdDep>(qh); h[1] = ld_u32_a2<LdDep>(qh + 4);
 #pragma unroll
             for (int q = 0; q < 4; ++q) sc[q] = ld_dep_u16(blk + 192 + n * 8 + 2 * q) >> (8 * (l0 >> 4));
             d = h2f(ld_dep_u16(blk + 208));
@@ -156,11 +155,6 @@ __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* W, OT* 
 // bytes - a half block's low nibbles and the high ones sixteen positions on - in each of two. Blocks are 34 and 18 bytes, so every
 // other one has its quants on a word boundary and the ones between two bytes behind one (a funnel shift). Needs rows of whole
 // groups (K a multiple of 128 / 64) on a 4-byte boundary. d * q is exact in FP32, one rounding to the output type.
-__device__ __forceinline__ uint32_t ld_dep_u32(const void* p) {
-    uint32_t v;
-    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
 template <int FMT, typename OT>
 __global__ void __launch_bounds__(256) dequant_32_kernel(const uint8_t* W, OT* out, long long total_units, int units_per_row, int row_bytes, int K) {
     constexpr int kBlock = FMT == kQ8_0 ? 34 : 18, kBlocks = FMT == kQ8_0 ? 4 : 2, kParts = FMT == kQ8_0 ? 4 : 2;

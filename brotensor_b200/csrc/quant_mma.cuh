@@ -144,7 +144,7 @@ __device__ __forceinline__ void qm_plain_rows(const uint8_t* W, const void* X, i
         for (int u = lane; u < (K >> 3); u += 32) {
             float w[8], v[8];
             uint4 raw[2];
-            decode8<FMT>(W + (size_t)n * row_bytes, u, w);
+            decode8<FMT, LdDep>(W + (size_t)n * row_bytes, u, w);
             qm_load_raw(X, x_dtype == B200Q_DT_F32, K, m, 8 * u, raw);
             qm_to_f32(raw, x_dtype, v);
 #pragma unroll

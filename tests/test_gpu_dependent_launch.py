@@ -55,3 +55,23 @@ def test_predecessor_writes_the_operands(fmt, N, K, M, ops_pdl):
     assert all(torch.equal(y, want[i & 1]) for i, y in enumerate(outs))
     assert all(torch.equal(y, want[c[0] & 1]) for c in captured for y in c[1:])
     assert ops.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,N,K,M,dtype", [(synth.Q5_K, 3000, 2560, 1, torch.float32), (synth.Q6_K, 700, 2304, 2, torch.float16), (synth.Q4_K, 1024, 4096, 6, torch.float16),
+                                             (synth.Q8_0, 700, 1024, 4, torch.bfloat16), (synth.Q4_0, 700, 1024, 20, torch.float32)])
+def test_predecessor_writes_operands_that_are_not_finite(fmt, N, K, M, dtype, ops_pdl):
+    """The FP32 loop that takes over for such activations reads the weights again, and no earlier."""
+    ops = ops_pdl
+    Ws = [torch.from_numpy(synth.make_blocks(fmt, N, K, seed=s)).cuda() for s in (1, 2)]
+    x = torch.from_numpy(synth.make_activations(M, K, seed=3)).to(dtype).cuda()
+    x[M // 2, 300] = float("inf")
+    ops.set_option("pdl", -1)
+    want = [ops.linear(fmt, W, x, N, out_dtype=torch.float32).view(torch.int32) for W in Ws]
+    ops.set_option("pdl", 0)
+    assert not torch.equal(*want)
+    W = torch.empty_like(Ws[0])
+    for i in range(40):
+        torch.bitwise_or(Ws[i & 1], 0, out=W)
+        assert torch.equal(ops.linear(fmt, W, x, N, out_dtype=torch.float32).view(torch.int32), want[i & 1])
+    assert ops.device_status() == 0
