@@ -54,16 +54,18 @@ constexpr int kXGroupStride = 272;
 // type: the type is a run-time switch around the load alone, so that the staging code exists once
 // per kernel instead of once per type (it used to be two thirds of the kernel's instructions, all of
 // them fetched cold at every launch).
+template <bool kDep = true>  // false: plain launches, the read-only path
 __device__ __forceinline__ void x_load_seg(const void* base, int x_dtype, int K, int idx, float (&v)[8]) {
     const int segs = K >> 3;
     const int m = idx / segs, seg = idx - m * segs;
     if (x_dtype == B200Q_DT_F32) {
         const float4* X = reinterpret_cast<const float4*>(static_cast<const float*>(base) + (size_t)m * K) + 2 * seg;
-        const float4 a = ld_dep_f4(X), b = ld_dep_f4(X + 1);
+        const float4 a = kDep ? ld_dep_f4(X) : __ldg(X), b = kDep ? ld_dep_f4(X + 1) : __ldg(X + 1);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
         v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     } else {
-        const uint4 q = ld_dep_u4(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + (size_t)m * K) + seg);
+        const uint4* X = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + (size_t)m * K) + seg;
+        const uint4 q = kDep ? ld_dep_u4(X) : __ldg(X);
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
         if (x_dtype == B200Q_DT_F16) {
 #pragma unroll

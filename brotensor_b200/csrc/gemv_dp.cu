@@ -80,13 +80,16 @@ __device__ __forceinline__ void x_store_seg(
 // Stages the activations as int16 with one power-of-two scale per 128-element group. A thread's
 // global loads go out four segments at a time before any of them is converted, so a long row
 // (K = 14336: 3.5 segments per thread) costs one load latency instead of one per segment.
-template <int FMT, bool kLean = false>
+// kDep: the launch may have started before its predecessor has finished, so the activations are read with ordinary loads behind
+// griddepcontrol.wait. Otherwise they take the read-only path, whose loads are not held in place by the code around them
+// (two rows, a plain launch, us, ordinary loads -> read-only: Q4_K 1024 x 8192 FP32 8.0 -> 6.4, 1024 x 12288 FP16 10.0 -> 8.5).
+template <int FMT, bool kLean, bool kDep>
 __device__ __forceinline__ void stage_x16(const StreamParams& p, uint32_t sbase, int tid, int nthreads) {
     const int total = (p.K >> 3) * p.M;  // K % 256 == 0, so a multiple of 32: whole warps are in or out
     if (kLean || total <= nthreads) {  // at most one segment per thread (K = 4096, one activation row)
         if (tid < total) {
             float v[8];
-            x_load_seg(p.X, kLean ? B200Q_DT_F32 : p.x_dtype, p.K, tid, v);
+            x_load_seg<kDep>(p.X, kLean ? B200Q_DT_F32 : p.x_dtype, p.K, tid, v);
             x_store_seg<FMT>(p, sbase, tid, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
         }
         return;
@@ -104,8 +107,8 @@ __device__ __forceinline__ void stage_x16(const StreamParams& p, uint32_t sbase,
             for (int u = 0; u < 4; ++u) {
                 const int idx = min(base + u * nthreads, total - 1), m = idx / segs, seg = idx - m * segs;
                 const float4* X = reinterpret_cast<const float4*>(static_cast<const float*>(p.X) + (size_t)m * p.K) + 2 * seg;
-                r[u][0] = ld_dep_f4(X);
-                r[u][1] = ld_dep_f4(X + 1);
+                r[u][0] = kDep ? ld_dep_f4(X) : __ldg(X);
+                r[u][1] = kDep ? ld_dep_f4(X + 1) : __ldg(X + 1);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -117,7 +120,8 @@ __device__ __forceinline__ void stage_x16(const StreamParams& p, uint32_t sbase,
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int idx = min(base + u * nthreads, total - 1), m = idx / segs, seg = idx - m * segs;
-                r[u] = ld_dep_u4(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.X) + (size_t)m * p.K) + seg);
+                const uint4* X = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.X) + (size_t)m * p.K) + seg;
+                r[u] = kDep ? ld_dep_u4(X) : __ldg(X);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -903,7 +907,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * NG * 32, 1) gemv_dp_ker
         // ---- producer of pipeline g. The predecessor may be what writes the weights (an upload, a repack):
         // unless the caller has said otherwise (early_w) they are read after griddepcontrol.wait.
         const int g = warp - kConsumers;
-        if (!p.early_w) {
+        if (MT == 1 && !p.early_w) {
             if (g < n_tiles) {  // the first stage's rows: into the L2 meanwhile
                 const TileRef tr = tile_ref<EXT>(p, row_begin + g * TR);
                 const int nrows = min(min(TR, row_end - (row_begin + g * TR)), tr.N - tr.row0);
@@ -979,7 +983,8 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * NG * 32, 1) gemv_dp_ker
     // calls of the candidate form so far, this one included (likewise stable while the launch runs)
     const unsigned int sh_cc = ((EXT & kExtShard) && p.sh_world > 0 && p.sh_topk > 0) ? *(volatile unsigned int*)&p.sh_state[2] + 1u : 0u;
     if ((EXT & kExtNorm) && MT == 1 && p.norm_gamma) stage_x16_norm<FMT>(p, sbase, tid, kConsumers * 32, norm_red);
-    else stage_x16<FMT, (EXT & kExtLean) != 0>(p, sbase, tid, kConsumers * 32);
+    else if (MT > 1 && !p.overlapped) stage_x16<FMT, (EXT & kExtLean) != 0, false>(p, sbase, tid, kConsumers * 32);
+    else stage_x16<FMT, (EXT & kExtLean) != 0, true>(p, sbase, tid, kConsumers * 32);
     TRACE_STAMP(tid == 0, 3);
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
 
@@ -1303,9 +1308,10 @@ static int launch_dp_k(const StreamParams& p_in, int grid, size_t smem, cudaStre
         B200Q_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    // (two to four rows: plain launches, under which reading the weights at once is no question)
+    // (two to four rows: plain launches unless pdl = 1, under which reading the weights at once is no question)
     p.early_w = MT > 1 || pdl_option() != 0;
-    B200Q_CUDA_TRY(launch_dep(MT == 1 ? pdl_option() >= 0 : pdl_option() > 0, kern, dim3((unsigned)grid), dim3((kConsumerWarps + 1) * NG * 32), smem, st, p));
+    p.overlapped = MT == 1 ? pdl_option() >= 0 : pdl_option() > 0;
+    B200Q_CUDA_TRY(launch_dep(p.overlapped != 0, kern, dim3((unsigned)grid), dim3((kConsumerWarps + 1) * NG * 32), smem, st, p));
     return B200Q_OK;
 }
 

@@ -35,6 +35,7 @@ struct StreamParams {
     int split_q, split_r;
     unsigned int wait_limit_us;  // bound of the device-side waits in microseconds (0: one second)
     int early_w;                 // 1: weights are read ahead of griddepcontrol.wait
+    int overlapped;              // 1: launched to start before the predecessor has finished
     int step_fill;               // 1: only the first stage of a pipeline is requested ahead of the activation loads
 #ifdef B200Q_TRACE
     unsigned long long* trace;  // trace builds: sixteen %globaltimer stamps per CTA of this launch

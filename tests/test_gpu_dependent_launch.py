@@ -75,3 +75,22 @@ def test_predecessor_writes_operands_that_are_not_finite(fmt, N, K, M, dtype, op
         torch.bitwise_or(Ws[i & 1], 0, out=W)
         assert torch.equal(ops.linear(fmt, W, x, N, out_dtype=torch.float32).view(torch.int32), want[i & 1])
     assert ops.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("pdl", [-1, 0, 1])
+def test_predecessor_writes_the_activations(pdl, M, ops_pdl):
+    """The integer-dot kernel in each launch form: plain launches read the activations on the read-only path, overlapped ones behind the wait."""
+    ops, fmt, N, K = ops_pdl, synth.Q4_K, 1024, 8192
+    W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=1)).cuda()
+    for dtype in (torch.float32, torch.float16):
+        xs = [torch.from_numpy(synth.make_activations(M, K, seed=s)).to(dtype).cuda() for s in (3, 4)]
+        ops.set_option("pdl", -1)
+        want = [ops.gemv(fmt, W, x, N) for x in xs]
+        ops.set_option("pdl", pdl)
+        x = torch.empty_like(xs[0])
+        for i in range(20):
+            torch.mul(xs[i & 1], 1.0, out=x)
+            assert torch.equal(ops.gemv(fmt, W, x, N), want[i & 1])
+    assert ops.device_status() == 0
