@@ -45,6 +45,7 @@ int launch_gemv_mb(int fmt, const void* W, const void* X, int x_dtype, const voi
 void mb_set_enabled(int v);
 int launch_gemv_hm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
                    int sms, cudaStream_t st, bool* taken);
+bool gemv_hm_takes(int fmt, const void* W, int x_dtype, int M, int N, int K);
 void hm_set_enabled(int v);
 int hm_get_enabled();
 size_t gemm_mm_workspace_bytes(int fmt, int x_dtype, int M, int N, int K);
@@ -122,6 +123,14 @@ static int dev_info(DevInfo** out) {
 }
 
 int* device_status_word(int dev) { return (dev >= 0 && dev < kMaxDev && g_dev[dev].ready.load(std::memory_order_acquire)) ? g_dev[dev].status : nullptr; }
+
+// Which kernel the thread's last linear call went to (option "last_kernel"): tests ask, since every route gives nearly the same numbers.
+enum { kRanPlain = 1, kRanStream, kRanDp, kRanXr, kRanI8, kRanHm, kRanMb, kRanMm, kRanTc };
+static thread_local int g_last_kernel = 0;
+static bool ran(bool taken, int kernel) {
+    if (taken) g_last_kernel = kernel;
+    return taken;
+}
 
 static int g_opt_gemv_path = 0;
 static int g_opt_gemm_path = 0;
@@ -242,6 +251,11 @@ int b200q_embedding_gather(int fmt, const void* table, const int32_t* idx, int B
     return launch_gather(fmt, table, idx, out, out_dtype, B, rows, K, static_cast<cudaStream_t>(stream));
 }
 
+static int gemv_plain(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K, cudaStream_t st) {
+    g_last_kernel = kRanPlain;
+    return launch_gemv_simple(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
+}
+
 // The streaming kernel for a decode GEMV of M <= 8 rows, by measurement on B200 (14336 x 4096 and
 // 4096 x 14336, us per launch): the integer-dot kernel's work grows with M, the warp-MMA kernel's
 // hardly does - Q4_K 8.1 / 12.8 / 16.1 / 21.9 at one to four rows against 16.7 / 18.3 / 19.9 / 21.3
@@ -254,23 +268,24 @@ static int gemv_streaming(DevInfo* d, int fmt, const void* W, const void* X, int
     const size_t smem = d->smem_optin - 1024;
     if (M >= 2) {  // Q8_0, K = 2048 / 4096: the integer tensor-core kernel streams at the one-row rate for any M <= 8
         if (int rc = launch_gemv_i8(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->status, st, taken)) return rc;
-        if (*taken) return B200Q_OK;
+        if (ran(*taken, kRanI8)) return B200Q_OK;
     }
     const bool mma_first = M >= (fmt == kQ8_0 ? 3 : 4);
     if (mma_first) {
         if (int rc = launch_gemv_stream(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, smem, d->status, st, taken)) return rc;
-        if (*taken) return B200Q_OK;
+        if (ran(*taken, kRanStream)) return B200Q_OK;
     }
     if (M == 1) {
         if (int rc = launch_gemv_xr(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->status, st, taken)) return rc;
-        if (*taken) return B200Q_OK;
+        if (ran(*taken, kRanXr)) return B200Q_OK;
     }
     if (M <= 4) {
         if (int rc = launch_gemv_dp(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, smem, d->status, st, taken, nullptr)) return rc;
-        if (*taken) return B200Q_OK;
+        if (ran(*taken, kRanDp)) return B200Q_OK;
     }
     if (!mma_first) {
         if (int rc = launch_gemv_stream(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, smem, d->status, st, taken)) return rc;
+        ran(*taken, kRanStream);
     }
     return B200Q_OK;
 }
@@ -314,14 +329,14 @@ int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* b
     if (g_opt_gemv_path == 0 && hm_wanted(fmt, x_dtype, M, N, K)) {
         bool taken = false;
         if (int rc = launch_gemv_hm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, st, &taken)) return rc;
-        if (taken) return B200Q_OK;
+        if (ran(taken, kRanHm)) return B200Q_OK;
     }
     if (g_opt_gemv_path == 0 && mb_wanted(fmt, M, N, K)) {
         bool taken = false;
         if (int rc = launch_gemv_mb(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->status, st, &taken)) return rc;
-        if (taken) return B200Q_OK;
+        if (ran(taken, kRanMb)) return B200Q_OK;
     }
-    if (!streaming_fmt(fmt)) return launch_gemv_simple(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
+    if (!streaming_fmt(fmt)) return gemv_plain(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
     // 0 = automatic, 1 = plain-load kernel, 2 = warp-MMA streaming kernel, 3 = integer-dot streaming kernel
     if (g_opt_gemv_path == 0) {
         bool taken = false;
@@ -338,7 +353,7 @@ int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* b
                 void* Y2 = static_cast<uint8_t*>(Y) + 4 * ys;
                 if (int rc = gemv_streaming(d, fmt, W, X2, x_dtype, bias, Y2, y_dtype, M - 4, N, K, st, &taken)) return rc;
                 if (taken) return B200Q_OK;
-                return launch_gemv_simple(fmt, W, X2, x_dtype, bias, Y2, y_dtype, M - 4, N, K, st);
+                return gemv_plain(fmt, W, X2, x_dtype, bias, Y2, y_dtype, M - 4, N, K, st);
             }
         }
     }
@@ -346,17 +361,17 @@ int b200q_gemv(int fmt, const void* W, const void* X, int x_dtype, const void* b
         bool taken = false;
         if (int rc = launch_gemv_dp(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->smem_optin - 1024, d->status, st, &taken, nullptr))
             return rc;
-        if (taken) return B200Q_OK;
+        if (ran(taken, kRanDp)) return B200Q_OK;
         return fail(B200Q_ERR_UNSUPPORTED, "gemv: shape (M %d, N %d, K %d, fmt %d) is outside the integer-dot kernel", M, N, K, fmt);
     }
     if (g_opt_gemv_path == 2) {
         bool taken = false;
         if (int rc = launch_gemv_stream(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, d->sms, d->smem_optin - 1024, d->status, st, &taken))
             return rc;
-        if (taken) return B200Q_OK;
+        if (ran(taken, kRanStream)) return B200Q_OK;
         return fail(B200Q_ERR_UNSUPPORTED, "gemv: shape (M %d, N %d, K %d, fmt %d) is outside the streaming kernel", M, N, K, fmt);
     }
-    return launch_gemv_simple(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
+    return gemv_plain(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, st);
 }
 
 int b200q_gemv_swiglu(int fmt, const void* W_gate, const void* W_up, const void* x, int x_dtype, void* y, int y_dtype,
@@ -371,7 +386,7 @@ int b200q_gemv_swiglu(int fmt, const void* W_gate, const void* W_up, const void*
     if (int rc = launch_gemv_dp_swiglu(fmt, W_gate, W_up, x, x_dtype, y, y_dtype, N, K, d->sms, d->smem_optin - 1024, d->status,
                                        static_cast<cudaStream_t>(stream), &taken))
         return rc;
-    if (!taken)
+    if (!ran(taken, kRanDp))
         return fail(B200Q_ERR_UNSUPPORTED, "gemv_swiglu: shape (N %d, K %d, fmt %d) or weight alignment is outside the streaming kernel", N, K, fmt);
     return B200Q_OK;
 }
@@ -391,7 +406,7 @@ int b200q_gemv_multi(int fmt, int n, const void* const* W, const int* N, void* c
         bool taken = false;
         if (int rc = launch_gemv_dp_multi(fmt, n, W, N, Y, bias, x, x_dtype, y_dtype, K, d->sms, d->smem_optin - 1024, d->status, st, &taken, nullptr, 0.f))
             return rc;
-        if (taken) return B200Q_OK;
+        if (ran(taken, kRanDp)) return B200Q_OK;
     }
     // shapes the grouped kernel does not take: one launch per matrix
     for (int s = 0; s < n; ++s)
@@ -416,7 +431,7 @@ int b200q_gemv_multi_rmsnorm(int fmt, int n, const void* const* W, const int* N,
     if (int rc = launch_gemv_dp_multi(fmt, n, W, N, Y, bias, x, x_dtype, y_dtype, K, d->sms, d->smem_optin - 1024, d->status,
                                       static_cast<cudaStream_t>(stream), &taken, gamma, eps))
         return rc;
-    if (!taken)
+    if (!ran(taken, kRanDp))
         return fail(B200Q_ERR_UNSUPPORTED, "gemv_multi_rmsnorm: shape (K %d, fmt %d) or weight alignment is outside the streaming kernel", K, fmt);
     return B200Q_OK;
 }
@@ -459,7 +474,7 @@ static int gemv_shard_impl(const char* name, int fmt, const void* W_shard, const
     if (int rc = launch_gemv_dp(fmt, W_shard, x, x_dtype, bias_shard, nullptr, B200Q_DT_F32, 1, rows, K, d->sms,
                                 d->smem_optin - 1024, d->status, static_cast<cudaStream_t>(stream), &taken, &sh))
         return rc;
-    if (!taken)
+    if (!ran(taken, kRanDp))
         return fail(B200Q_ERR_UNSUPPORTED, "%s: shape (rows %d, K %d, fmt %d) or weight alignment is outside the streaming kernel", name, rows, K, fmt);
     return B200Q_OK;
 }
@@ -496,13 +511,12 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Up to sixteen rows of 16-bit activations of a matrix of few rows: two passes of the small-batch GEMV (4096 x 4096 Q4_K 13 us
     // against 20, 2560 x 6912 Q4_K 20 against 31, 4096 x 14336 Q5_K 42 against 60 of the kernels below).
-    const bool two_passes = g_opt_gemm_path == 0 && g_opt_gemv_path == 0 && M > 8 && M <= 16 && N <= 8192 && K % 256 == 0 && fmt != kQ6_KP &&
-                            hm_get_enabled() && hm_wanted(fmt, x_dtype, 8, N, K) &&
-                            (fmt == kQ6_K || aligned(W, 16));
+    const bool two_passes = g_opt_gemm_path == 0 && g_opt_gemv_path == 0 && M > 8 && M <= 16 && N <= 8192 && hm_wanted(fmt, x_dtype, 8, N, K) &&
+                            gemv_hm_takes(fmt, W, x_dtype, 8, N, K);
     if (!two_passes && g_opt_gemm_path == 0 && mm_wanted(fmt, M)) {
         bool taken = false;
         if (int rc = launch_gemm_mm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, ws, ws_bytes, d->sms, st, &taken)) return rc;
-        if (taken) {
+        if (ran(taken, kRanMm)) {
             if (fmt_slot(fmt) >= 0) d->tc_calls[fmt_slot(fmt)].fetch_add(1);
             return B200Q_OK;
         }
@@ -527,7 +541,7 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
         bool taken = false;
         if (int rc = launch_gemm_tc(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, ws, ws_bytes, d->sms, d->status, st, &taken))
             return rc;
-        if (taken) {
+        if (ran(taken, kRanTc)) {
             d->tc_calls[fmt_slot(fmt)].fetch_add(1);
             return B200Q_OK;
         }
@@ -619,6 +633,7 @@ int b200q_get_option(const char* key, int* out) {
     else if (!strcmp(key, "gemm_pair")) *out = gemm_get_pair();
     else if (!strcmp(key, "gemm_split")) *out = gemm_get_split();
     else if (!strcmp(key, "wait_limit_us")) *out = dp_get_wait_limit_us();
+    else if (!strcmp(key, "last_kernel")) *out = g_last_kernel;
     else return fail(B200Q_ERR_BAD_ARG, "get_option: unknown key '%s'", key);
     return B200Q_OK;
 }

@@ -393,7 +393,7 @@ static int launch_hm(const HmParams& p, int grid, size_t smem, cudaStream_t st) 
 }
 
 template <int FMT>
-static int launch_hm_f(HmParams& p, bool bf, int sms, cudaStream_t st, bool* taken) {
+static int launch_hm_f(HmParams& p, bool bf, int sms, cudaStream_t st) {
     using F = QmFmt<FMT>;
     p.row_bytes = p.nblk * F::bytes;
     int grid = stream_get_option(3) > 0 ? stream_get_option(3) : sms;
@@ -403,47 +403,53 @@ static int launch_hm_f(HmParams& p, bool bf, int sms, cudaStream_t st, bool* tak
     const int rows = p.row_q + (p.row_r ? 1 : 0), tiles = (rows + kQmTile - 1) / kQmTile;
     const int iters = (tiles + kHmMaxTiles - 1) / kHmMaxTiles;
     p.mt = (tiles + iters - 1) / iters;
-    // as many blocks per stage as there are warps left for a tile, the stages of a row as even as they come
-    int kg = kHmMaxWarps / p.mt;
-    p.k_stages = (p.nblk + kg - 1) / kg;
-    p.kg = kg = (p.nblk + p.k_stages - 1) / p.k_stages;
-    // Activations resident, no stage barrier: 14336 x 4096 Q4_K (8 steps) 18.9 -> 17.2 us, 32000 x 4096 (16) 37.5 -> 31.5, 4096 x 14336 one row (7)
-    // 17.5 -> 16.9; but the start waits for all of X, so short runs lose: 4096 x 4096 (2 steps) 6.5 -> 7.2, 2560 x 6912 (4) 8.8 -> 9.3.
-    if ((long long)p.M * p.K <= kHmResident && iters * p.k_stages >= 6) {
-        const size_t x = (size_t)p.nblk * p.M * 512, red = 2 * (size_t)(kg - 1) * p.mt * 512, tail = red > 3584 ? red : 3584, budget = 227 * 1024 - 1024 - 256;
-        const size_t tile = (size_t)p.mt * kg * kQmTile * F::stride;
-        p.n_stages = kHmMaxStages;
-        while (p.n_stages > 2 && p.n_stages * tile + x + tail > budget) --p.n_stages;
-        if (p.n_stages * tile + x + tail <= budget) {
-            p.off_x = (int)(p.n_stages * tile);
-            p.off_red = p.off_x + (int)x;
-            *taken = true;
-            const size_t smem = (size_t)p.off_red + tail + 128;
-            return bf ? launch_hm<FMT, true, true>(p, grid, smem, st) : launch_hm<FMT, false, true>(p, grid, smem, st);
+    // As many blocks per stage as there are warps left for a tile and as leave room for two stages, the stages of a row as even as they
+    // come. (Eight rows of 1024 x 12288 Q8_0 have room for 12 blocks, not 16: 9.0 us, and 16 to 25 on the kernels that took such calls before;
+    // holding out for three stages instead costs 2 to 24 % on K = 2560 .. 14336 and gains 2 to 6 % on a few shapes.)
+    const size_t budget = 227 * 1024 - 1024 - 256;
+    for (int most = kHmMaxWarps / p.mt;; --most) {
+        p.k_stages = (p.nblk + most - 1) / most;
+        p.kg = (p.nblk + p.k_stages - 1) / p.k_stages;
+        // sums of the tile's warps; rows past M of the last block's activations are read, not used: up to 7 x 512 bytes past the stage
+        const size_t red = (size_t)(p.kg - 1) * p.mt * 512, tile = (size_t)p.mt * p.kg * kQmTile * F::stride;
+        // Activations resident, no stage barrier: 14336 x 4096 Q4_K (8 steps) 18.9 -> 17.2 us, 32000 x 4096 (16) 37.5 -> 31.5, 4096 x 14336 one row (7)
+        // 17.5 -> 16.9; but the start waits for all of X, so short runs lose: 4096 x 4096 (2 steps) 6.5 -> 7.2, 2560 x 6912 (4) 8.8 -> 9.3.
+        if ((long long)p.M * p.K <= kHmResident && iters * p.k_stages >= 6) {
+            const size_t x = (size_t)p.nblk * p.M * 512, tail = 2 * red > 3584 ? 2 * red : 3584;
+            p.n_stages = kHmMaxStages;
+            while (p.n_stages > 2 && p.n_stages * tile + x + tail > budget) --p.n_stages;
+            if (p.n_stages * tile + x + tail <= budget) {
+                p.off_x = (int)(p.n_stages * tile);
+                p.off_red = p.off_x + (int)x;
+                const size_t smem = (size_t)p.off_red + tail + 128;
+                return bf ? launch_hm<FMT, true, true>(p, grid, smem, st) : launch_hm<FMT, false, true>(p, grid, smem, st);
+            }
         }
+        const size_t tail = red > 3584 ? red : 3584;
+        p.off_x = (int)tile;
+        p.stage_bytes = (p.off_x + p.kg * p.M * 512 + 127) & ~127;
+        p.n_stages = kHmMaxStages;
+        while (p.n_stages > 2 && (size_t)p.n_stages * p.stage_bytes + tail > budget) --p.n_stages;
+        if ((size_t)p.n_stages * p.stage_bytes + tail > budget && most > 1) continue;  // (one block per stage fits: 2 x 39 KB at most)
+        p.off_red = p.n_stages * p.stage_bytes;
+        const size_t smem = (size_t)p.off_red + tail + 128;
+        return bf ? launch_hm<FMT, true, false>(p, grid, smem, st) : launch_hm<FMT, false, false>(p, grid, smem, st);
     }
-    p.off_x = p.mt * kg * kQmTile * F::stride;
-    p.stage_bytes = (p.off_x + kg * p.M * 512 + 127) & ~127;
-    // (rows past M of the last block's activations are read, not used: up to 7 x 512 bytes past the stage)
-    const size_t red = (size_t)(kg - 1) * p.mt * 512, budget = 227 * 1024 - 1024 - 256;
-    const size_t tail = red > 3584 ? red : 3584;
-    p.n_stages = kHmMaxStages;
-    while (p.n_stages > 2 && (size_t)p.n_stages * p.stage_bytes + tail > budget) --p.n_stages;
-    if ((size_t)p.n_stages * p.stage_bytes + tail > budget) return B200Q_OK;
-    p.off_red = p.n_stages * p.stage_bytes;
-    *taken = true;
-    const size_t smem = (size_t)p.off_red + tail + 128;
-    return bf ? launch_hm<FMT, true, false>(p, grid, smem, st) : launch_hm<FMT, false, false>(p, grid, smem, st);
 }
 
-// Launches the kernel when it takes the call (*taken = true): FP16 or BF16 activations, K a multiple of 256, weights on a 16-byte boundary
+// The calls it takes, and takes in every case: FP16 or BF16 activations, 1..8 rows, K a multiple of 256, weights on a 16-byte boundary
 // (Q6_K: any even address).
+bool gemv_hm_takes(int fmt, const void* W, int x_dtype, int M, int N, int K) {
+    if (!g_opt_hm || x_dtype == B200Q_DT_F32 || M < 1 || M > 8 || N < 1 || K < 256 || K % 256 != 0) return false;
+    if (fmt == kQ6_K) return true;
+    return (fmt == kQ4_K || fmt == kQ5_K || fmt == kQ8_0 || fmt == kQ4_0) && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+}
+
 int launch_gemv_hm(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M, int N, int K,
                    int sms, cudaStream_t st, bool* taken) {
-    *taken = false;
+    *taken = gemv_hm_takes(fmt, W, x_dtype, M, N, K);
+    if (!*taken) return B200Q_OK;
     const bool bf = x_dtype == B200Q_DT_BF16;
-    if (!g_opt_hm || x_dtype == B200Q_DT_F32 || M < 1 || M > 8 || N < 1 || K < 256 || K % 256 != 0) return B200Q_OK;
-    if (fmt != kQ6_K && (reinterpret_cast<uintptr_t>(W) & 15) != 0) return B200Q_OK;
     HmParams p = {};
     p.W = static_cast<const uint8_t*>(W);
     p.X = static_cast<const uint8_t*>(X);
@@ -455,13 +461,12 @@ int launch_gemv_hm(int fmt, const void* W, const void* X, int x_dtype, const voi
     p.y_dtype = y_dtype;
     p.nblk = K / 256;
     switch (fmt) {
-        case kQ4_K: return launch_hm_f<kQ4_K>(p, bf, sms, st, taken);
-        case kQ5_K: return launch_hm_f<kQ5_K>(p, bf, sms, st, taken);
-        case kQ6_K: return launch_hm_f<kQ6_K>(p, bf, sms, st, taken);
-        case kQ8_0: return launch_hm_f<kQ8_0>(p, bf, sms, st, taken);
-        case kQ4_0: return launch_hm_f<kQ4_0>(p, bf, sms, st, taken);
+        case kQ4_K: return launch_hm_f<kQ4_K>(p, bf, sms, st);
+        case kQ5_K: return launch_hm_f<kQ5_K>(p, bf, sms, st);
+        case kQ6_K: return launch_hm_f<kQ6_K>(p, bf, sms, st);
+        case kQ8_0: return launch_hm_f<kQ8_0>(p, bf, sms, st);
+        default: return launch_hm_f<kQ4_0>(p, bf, sms, st);
     }
-    return B200Q_OK;
 }
 
 }  // namespace b200q

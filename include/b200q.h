@@ -303,6 +303,9 @@ int b200q_device_status(int* status_out);
  *   "gemv_lean"   0 = never take the trimmed instantiation of the integer-dot kernel (FP32 in and out, no bias)
  *   "wait_limit_us" bound of the decode kernels' device-side waits (stage barriers, peer arrival) in
  *                 microseconds; 0 = one second. Tests shorten it to see a wait run out.
+ *   "last_kernel" (read only) the kernel of the calling thread's last linear call, its last pass: 1 plain-load GEMV, 2 warp-MMA
+ *                 streaming, 3 integer-dot, 4 activation-resident, 5 integer tensor-core (2..8 rows), 6 "gemv_hm", 7 "gemv_mb",
+ *                 8 "gemm_mm", 9 tcgen05 GEMM; 0 = none yet
  * Returns B200Q_ERR_BAD_ARG for an unknown key.
  */
 int b200q_set_option(const char* key, int value);

@@ -3,14 +3,17 @@
 FP32: exact products, sums of a few hundred FP32 terms (at most sqrt(K / 32 + 16) * 2^-24 < 2e-6 over a row for K <= 14336), so that is the bound.
 Sizes: one row, ragged tiles of 16, fewer rows than SMs, several row tiles per CTA, several passes over a CTA's rows, K of one block, of
 an odd number of blocks (Q6_K rows that start on any even byte) and of more blocks than a CTA has warps."""
+import ctypes
+
 import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 
 import oracle
-from brotensor_b200 import synth
+from brotensor_b200 import _capi, synth
 
+HM, MB, MM = 6, 7, 8  # what the option "last_kernel" calls them
 FMTS = [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0, synth.Q4_0]
 SHAPES = [(1, 256), (15, 512), (37, 768), (300, 6912), (2373, 1024), (40, 14336), (20000, 256)]
 DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
@@ -24,6 +27,12 @@ def ops_raw():
         ops.set_option(key, 1)
     ops.set_option("pdl", 0)
     assert ops.device_status() == 0
+
+
+def _last_kernel():
+    v = ctypes.c_int(0)
+    _capi.check(_capi.lib().b200q_get_option(b"last_kernel", ctypes.byref(v)))
+    return v.value
 
 
 def _operands(fmt, N, K, M, dtype):
@@ -49,6 +58,7 @@ def test_decode_rows(fmt, N, K, ops_raw):
             if kernel == "gemv_mb" and fmt in (synth.Q4_K, synth.Q8_0):
                 continue
             y = ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32)
+            assert _last_kernel() == (HM if kernel == "gemv_hm" else MB), (kernel, M, dtype)
             assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (kernel, M, dtype)
             assert torch.equal(y, ops.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32))  # fixed order of additions
             for early in (-1, 1):
@@ -71,6 +81,21 @@ def test_a_few_dozen_tokens(fmt, N, K, ops_raw):
         y = ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32)
         assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (M, dtype)
         assert torch.equal(y, ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,N,K", [(synth.Q8_0, 640, 14336), (synth.Q8_0, 640, 4096), (synth.Q6_K, 1024, 12288), (synth.Q5_K, 300, 8192), (synth.Q4_K, 40, 4096)])
+def test_matrices_of_few_rows_and_many_activations(fmt, N, K, ops_raw):
+    """Blocks of long rows beside eight activation rows: as many per stage as fit, on the same kernel."""
+    ops = ops_raw
+    for M in (6, 7, 8, 9, 16):
+        W, x, b, want = _operands(fmt, N, K, M, "f16")
+        ops.set_option("gemv_i8", 0)  # (K = 4096 of Q8_0 / Q4_K has another kernel for eight rows)
+        ops.set_option("gemv_hm", 2)
+        y = ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32)
+        ops.set_option("gemv_i8", 1)
+        assert _last_kernel() == HM, M
+        assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, M
 
 
 @pytest.mark.gpu
