@@ -295,7 +295,8 @@ static int gemv_streaming(DevInfo* d, int fmt, const void* W, const void* X, int
 // rate, so the lines lie where the older kernels' times cross theirs (us, old -> gemv_hm, FP16, overlapped launches):
 //   Q4_K   M = 2: 1024 x 4096 4.6 -> 3.7, 6912 x 2560 7.7 -> 6.3, 4096 x 14336 15.9 -> 17.9, 14336 x 4096 12.5 -> 19.1
 //          M = 6: 4096 x 4096 10.6 -> 6.5, 4096 x 14336 49 -> 18.5, 2560 x 6912 22 -> 9.6, 14336 x 4096 (integer MMA) 18.1 -> 19.0
-//   Q6_K   M = 2: 1024 x 4096 4.9 -> 4.3, 4096 x 4096 7.7 -> 8.3; M = 6: 10.3 -> 8.7, 4096 x 14336 43 -> 25, 14336 x 4096 22 -> 25
+//   Q6_K   M = 2: 1024 x 4096 5.0 -> 4.5, 2048 x 4096 5.9 -> 5.5, 1024 x 8192 7.2 -> 7.2, 2048 x 8192 8.3 -> 8.8, 2048 x 14336 12.7 -> 14.3,
+//          4096 x 4096 7.7 -> 8.3; M = 3: 2048 x 14336 16.9 -> 14.7; M = 6: 10.3 -> 8.7, 4096 x 14336 43 -> 25, 14336 x 4096 22 -> 25
 //   Q8_0   M = 2: 4096 x 4096 10.9 -> 7.7, 4096 x 14336 19.8 -> 21.6; M = 6: 11.4 -> 7.9, 43.6 -> 22, 14336 x 4096 18.8 -> 21.9
 // Rows of Q6_K that are not whole runs of eight blocks, Q5_K and Q4_0 had the plain-load kernel (2560 x 6912, M = 1: 20.8 -> 11.6,
 // 24.8 -> 10.2, 19.8 -> 8.0); from M = 1, 2 and many rows gemv_mb is the faster of the two for the 4- and 5-bit formats (14336 x 4096
@@ -308,7 +309,7 @@ static bool hm_wanted(int fmt, int x_dtype, int M, int N, int K) {
         case kQ5_K: return M > 2 || few;
         case kQ4_0: return M > 2 || N <= 16384;
         case kQ4_K: return M == 2 ? K <= 4096 && (long long)N * K <= 18000000 : M > 2 && (few || (M >= 4 && K != 2048 && K != 4096));
-        case kQ6_K: return K % kQ6RunElems != 0 ? M > 2 || few : M >= 4 ? few : M >= 2 && N <= 2048;
+        case kQ6_K: return K % kQ6RunElems != 0 ? M > 2 || few : M >= 4 ? few : M >= 2 && N <= 2048 && (M > 2 || (long long)N * K <= 2048 * 4096);
         case kQ8_0: return M >= 2 && (few ? M > 2 || K <= 8192 : M > 2 && K != 2048 && K != 4096 && N <= 16384);
     }
     return false;

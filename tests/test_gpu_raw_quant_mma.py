@@ -13,7 +13,7 @@ torch = pytest.importorskip("torch")
 import oracle
 from brotensor_b200 import _capi, synth
 
-HM, MB, MM = 6, 7, 8  # what the option "last_kernel" calls them
+DP, HM, MB, MM = 3, 6, 7, 8  # what the option "last_kernel" calls them
 FMTS = [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0, synth.Q4_0]
 SHAPES = [(1, 256), (15, 512), (37, 768), (300, 6912), (2373, 1024), (40, 14336), (20000, 256)]
 DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
@@ -96,6 +96,16 @@ def test_matrices_of_few_rows_and_many_activations(fmt, N, K, ops_raw):
         ops.set_option("gemv_i8", 1)
         assert _last_kernel() == HM, M
         assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, M
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K,M,kernel", [(2048, 4096, 2, HM), (2048, 8192, 2, DP), (1024, 14336, 2, DP), (2048, 14336, 3, HM)])
+def test_two_rows_of_q6k(N, K, M, kernel, ops_raw):
+    """Two rows of a longer Q6_K matrix are the integer-dot kernel's."""
+    W, x, b, want = _operands(synth.Q6_K, N, K, M, "f16")
+    y = ops_raw.gemv(synth.Q6_K, W, x, N, bias=b, out_dtype=torch.float32)
+    assert _last_kernel() == kernel
+    assert oracle.rel_l2(y.cpu().numpy(), want) < (2e-6 if kernel == HM else 2e-3)  # (15-bit fixed point in the other)
 
 
 @pytest.mark.gpu
