@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
     if (__any_sync(0xffffffffu, any)) {
         __syncthreads();  // the stores above come first
         for (int m = 0; m < p.tokens; ++m)
-            if (p.nonfinite[m]) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, p.N, p.K, p.row_bytes, row_begin, n_rows);
+            if (p.nonfinite[m]) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, 1u, p.N, p.K, p.row_bytes, row_begin, n_rows);
     }
 }
 

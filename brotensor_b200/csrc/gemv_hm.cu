@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
     }
     __syncthreads();
     if (nonfinite)
-        for (int m = 0; m < p.M; ++m) qm_plain_rows<FMT>(p.W, p.X, BF ? B200Q_DT_BF16 : B200Q_DT_F16, p.bias, p.Y, p.y_dtype, m, p.N, p.K, p.row_bytes, row_begin, n_rows);
+        qm_plain_rows<FMT>(p.W, p.X, BF ? B200Q_DT_BF16 : B200Q_DT_F16, p.bias, p.Y, p.y_dtype, 0, (1u << p.M) - 1u, p.N, p.K, p.row_bytes, row_begin, n_rows);
 }
 
 // ---- host side ------------------------------------------------------------------------------------------

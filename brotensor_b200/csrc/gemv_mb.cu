@@ -7,12 +7,13 @@
 //   * Weights stay integers. A 16-row x 32-k piece of the blocks is the A operand of mma.sync.m16n8k32 (Q6_K, whose
 //     scales cover 16 elements: m16n8k16), unpacked with one to four logic operations per four weights; block and
 //     sub-block scales are applied to the integer sums.
-//   * Activations are fixed point with one power-of-two scale per 256 elements and row, cut into signed bytes ("planes"):
-//     four of them (30 bits) or, for five to eight rows of 16-bit activations, three (22 bits, which hold an FP16 or
-//     BF16 value exactly down to 2^-11 of the block's largest). The MMA's eight columns are (plane, row) pairs - four
-//     planes of two rows, two planes of four, or one plane of eight - so one to two rows need ONE MMA per k-step, three to
-//     four two, five to eight three or four. Integer sums are exact; a result's error is that of a few hundred
-//     FP32 additions.
+//   * Activations are fixed point with one power-of-two scale per 256 elements and row, cut into signed bytes ("planes"). The
+//     MMA's eight columns are (plane, row) pairs: eight planes of one FP32 row (62 bits, in which a value above 2^-36 of the block's
+//     largest is exact), four planes of two rows (30 bits: FP32 values are exact down to 2^-6 of the largest, FP16 ones to 2^-19, BF16
+//     ones to 2^-22), two of four or one of eight. So one to two rows need ONE MMA per k-step, three to four two, five to eight
+//     four. Integer sums are exact; a result's error is that of a few hundred FP32 additions, as long as what the planes leave out is
+//     small beside the bulk of a sub-block's activations and not only beside the largest (qm_sub_block_lost); a row where it is not (a
+//     channel some thousand times the others, in FP32), or of magnitudes outside 2^-90 .. 2^97, takes the plain loop below.
 //   * A warp owns one 256-element block column of the weight rows ("its block") for a whole phase of the launch: the B
 //     fragments of that block stay in registers (16 per MMA column set). Up to sixteen warps cover K = 4096; longer rows run in
 //     phases over the CTA's rows, shorter ones with several row groups side by side.
@@ -27,7 +28,7 @@
 // Measured (one row, us, plain-load kernel -> this one): Q5_K 14336 x 4096 39.8 -> 17.1, 4096 x 4096 16.9 -> 7.4, 4096 x 14336 50.6 -> 19.5; Q4_0 29.5 -> 17.6,
 // 13.1 -> 7.1, 40.4 -> 19.4; Q6_K 2560 x 6912 20.8 -> 12.4. It runs at half of the memory's rate for one row: 58 instructions per k-step of
 // 16 x 32, of which the kernel's own work is about 25 and the rest is waiting for the others at a tile's end.
-// Activations that are not finite take a plain FP32 loop at the end of the launch (qm_plain_rows).
+// Rows of activations that are not finite or not held take a plain FP32 loop at the end of the launch (qm_plain_rows).
 //
 // Takes the place of brotensor's decode GEMVs (src/cuda/q4k.cu:159-224, q6k.cu:117-176, q8_0.cu:75-138) and of the
 // per-row loop of its batched ops for small B (q4k.cu:413-418).
@@ -80,10 +81,10 @@ template <int NB>
 struct MbX {
     uint2 b[8][NB];   // B fragments of the eight k-steps
     float mn[NB][2];  // B fragments of the mins' MMA: pieces of the sub-block sums t and t + 4 of the lane's column
-    float cs[2];      // 2^-e of the accumulator columns 2t and 2t + 1
+    float cs[2];      // what the accumulator columns 2t and 2t + 1 count: 2^-e, with eight planes the highest plane's 2^(24-e)
 };
 
-// One block column of a 16-row tile: v = this warp's share of (row g, columns 2t, 2t + 1), (row g + 8, same), the
+// One block column of a 16-row tile (FP32 factors are applied in an order that keeps products of sums and block scales in range): v = this warp's share of (row g, columns 2t, 2t + 1), (row g + 8, same), the
 // planes that sit in different column sets already combined. ra, rb: rows g and g + 8.
 template <int FMT, int MC, int NB>
 __device__ __forceinline__ void mb_block(const QmRow& ra, const QmRow& rb, int t, const MbX<NB>& x, float (&v)[4]) {
@@ -136,10 +137,10 @@ __device__ __forceinline__ void mb_block(const QmRow& ra, const QmRow& rb, int t
             }
         }
         const float dA = h2f(hA.x & 0xFFFFu), dB = h2f(hB.x & 0xFFFFu), mA = h2f(hA.x >> 16), mB = h2f(hB.x >> 16);
-        v[0] = fmaf(dA * x.cs[0], f[0], -(mA * fm[0]));
-        v[1] = fmaf(dA * x.cs[1], f[1], -(mA * fm[1]));
-        v[2] = fmaf(dB * x.cs[0], f[2], -(mB * fm[2]));
-        v[3] = fmaf(dB * x.cs[1], f[3], -(mB * fm[3]));
+        v[0] = fmaf(dA * f[0], x.cs[0], -(mA * fm[0]));
+        v[1] = fmaf(dA * f[1], x.cs[1], -(mA * fm[1]));
+        v[2] = fmaf(dB * f[2], x.cs[0], -(mB * fm[2]));
+        v[3] = fmaf(dB * f[3], x.cs[1], -(mB * fm[3]));
     } else if constexpr (FMT == kQ6_K) {
         int is[NB][4];
 #pragma unroll
@@ -192,10 +193,10 @@ __device__ __forceinline__ void mb_block(const QmRow& ra, const QmRow& rb, int t
 #pragma unroll
             for (int i = 0; i < 4; ++i) f[i] = fmaf(f[i], kStep, (float)is[nb][i]);
         const float dA = h2f((ls32(ra.p + 208) >> ra.sh) & 0xFFFFu) * 0.25f, dB = h2f((ls32(rb.p + 208) >> rb.sh) & 0xFFFFu) * 0.25f;
-        v[0] = dA * x.cs[0] * f[0];
-        v[1] = dA * x.cs[1] * f[1];
-        v[2] = dB * x.cs[0] * f[2];
-        v[3] = dB * x.cs[1] * f[3];
+        v[0] = dA * f[0] * x.cs[0];
+        v[1] = dA * f[1] * x.cs[1];
+        v[2] = dB * f[2] * x.cs[0];
+        v[3] = dB * f[3] * x.cs[1];
     } else {
         // Q4_0: a scale per 32 elements. The MMA starts from the bits of 1.5 * 2^23, so its integer result (at most
         // 2^19) read as a float is that number plus the sum: one subtraction instead of a conversion.
@@ -238,19 +239,17 @@ __device__ __forceinline__ void mb_block(const QmRow& ra, const QmRow& rb, int t
 }
 
 // Fixed point and byte planes of the warp's block: x rows 0 .. M-1, elements [256 blk, 256 blk + 256), into fragments.
-// `scratch`: 2304 bytes of shared memory of the warp's own. Returns false when a value is not finite.
+// `scratch`: 2304 bytes of shared memory of the warp's own. Returns the rows (bits) that are not finite or not held closely enough.
 template <int FMT, int MC, int NB>
-__device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t scratch, int lane, MbX<NB>& x) {
+__device__ __forceinline__ uint32_t mb_stage_x(const MbParams& p, int blk, uint32_t scratch, int lane, MbX<NB>& x) {
     constexpr int kPlanes = 8 * NB / MC;
-    constexpr int kBits = kPlanes == 4 ? 29 : 21;  // the largest value lies in [2^kBits, 2^(kBits + 1))
-    constexpr uint32_t kBias = kPlanes == 4 ? 0x80808080u : 0x00808080u;
+    static_assert(kPlanes == 4 || kPlanes == 8, "planes");
     const int g = lane >> 2, t = lane & 3;
-    // one column set per plane: three for 16-bit activations, four for FP32 (launch_mb_f)
-    const bool f32 = MC == 8 ? NB == 4 : p.x_dtype == B200Q_DT_F32;
-    constexpr int kBatch = (MC == 8 && NB == 4) ? 4 : MC;  // rows whose loads are in flight together (registers)
-    uint32_t w[MC][kPlanes][2];                            // byte planes of the lane's eight elements
+    const bool f32 = p.x_dtype == B200Q_DT_F32;
+    constexpr int kBatch = MC == 8 ? 4 : MC;  // rows whose loads are in flight together (registers)
+    uint32_t w[MC][kPlanes][2];               // byte planes of the lane's eight elements
     float s0 = 0.f, s1 = 0.f;  // sums of x over sub-blocks t and t + 4, row of this lane's column
-    bool finite = true;
+    uint32_t left = 0;
     x.cs[0] = x.cs[1] = 0.f;
 #pragma unroll
     for (int m0 = 0; m0 < MC; m0 += kBatch) {
@@ -263,24 +262,49 @@ __device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t 
             const int m = m0 + i;
             if (m < p.M) {
                 float f[8];
-                qm_to_f32(raw[i], MC == 8 ? (f32 ? B200Q_DT_F32 : (p.x_dtype == B200Q_DT_F16 ? B200Q_DT_F16 : B200Q_DT_BF16)) : p.x_dtype, f);
-                uint32_t top = 0;
+                qm_to_f32(raw[i], p.x_dtype, f);
+                uint32_t mine = 0;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) top = max(top, __float_as_uint(f[k]) & 0x7FFFFFFFu);
-                top = __reduce_max_sync(0xffffffffu, top);
-                finite &= top < 0x7F800000u;
-                int e = kBits + 127 - (int)(top >> 23);
-                e = top == 0 ? 0 : max(-126, min(126, e));
-                const float s = __uint_as_float((uint32_t)(e + 127) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
-                uint32_t u[8];
+                for (int k = 0; k < 8; ++k) mine = max(mine, __float_as_uint(f[k]) & 0x7FFFFFFFu);
+                const uint32_t top = __reduce_max_sync(0xffffffffu, mine);
+                // 2^-90 .. 2^97: scales, sums of x and their pieces stay in FP32's range
+                const bool in_range = top - 0x12800000u < 0x70000000u - 0x12800000u;
+                // the largest value lies in [2^29, 2^30)
+                const int e = in_range ? 29 + 127 - (int)(top >> 23) : 0;
+                const float s = __uint_as_float((uint32_t)(e + 127) << 23), inv = __uint_as_float((uint32_t)(127 - e + (kPlanes == 8 ? 24 : 0)) << 23);
+                uint32_t u[kPlanes / 4][8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) u[k] = (uint32_t)__float2int_rn(f[k] * s) + kBias;
+                for (int k = 0; k < 8; ++k) {
+                    const float v = f[k] * s;
+                    const int hi = __float2int_rn(v);
+                    if constexpr (kPlanes == 8) {
+                        const int lo = __float2int_rn((v - (float)hi) * 2147483648.0f);
+                        const unsigned long long b = ((unsigned long long)(unsigned int)hi << 32) + (unsigned long long)(2LL * lo) + 0x8080808080808080ull;
+                        u[0][k] = (uint32_t)b;
+                        u[1][k] = (uint32_t)(b >> 32);
+                    } else {
+                        u[0][k] = (uint32_t)hi + 0x80808080u;
+                    }
+                }
+                // Where every eight neighbours reach 2^-6 of the block's largest (eight planes: 2^-30), the planes hold enough of them; elsewhere it
+                // is looked at closely.
+                if (__any_sync(0xffffffffu, mine + ((kPlanes == 8 ? 30u : 6u) << 23) < top)) {
+                    float err2 = 0.f;  // of eight planes at most 2^-32 each
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float err = kPlanes == 8 ? 2.3283064365386963e-10f : f[k] * s - (float)__float2int_rn(f[k] * s);
+                        err2 = fmaf(err, err, err2);
+                    }
+                    if (qm_sub_block_lost(f, s, err2)) left |= 1u << m;
+                }
+                if (top != 0 && !in_range) left |= 1u << m;
 #pragma unroll
                 for (int pl = 0; pl < kPlanes; ++pl)
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint32_t a = __byte_perm(u[4 * h], u[4 * h + 1], pl | ((4 + pl) << 4)), b = __byte_perm(u[4 * h + 2], u[4 * h + 3], pl | ((4 + pl) << 4));
-                        w[m][pl][h] = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+                        const uint32_t* q = &u[pl / 4][4 * h];
+                        const uint32_t sel = (pl & 3) | ((4 + (pl & 3)) << 4);
+                        w[m][pl][h] = __byte_perm(__byte_perm(q[0], q[1], sel), __byte_perm(q[2], q[3], sel), 0x5410) ^ 0x80808080u;
                     }
                 if (((2 * t) & (MC - 1)) == m) x.cs[0] = inv;
                 if (((2 * t + 1) & (MC - 1)) == m) x.cs[1] = inv;
@@ -298,7 +322,7 @@ __device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t 
         }
     }
     if constexpr (QmFmt<FMT>::mins) {
-        // three pieces of 11 bits, piece i divided by 256^i because plane i of the columns counts 256^i times
+        // three pieces of 11 bits; plane i of four counts 256^i times (of eight: the highest once, the next 1 / 256), so a piece is divided by that
         float pc[4][2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -306,8 +330,8 @@ __device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t 
             const float a = __uint_as_float(__float_as_uint(s) & 0xFFFFE000u), r = s - a;
             const float b = __uint_as_float(__float_as_uint(r) & 0xFFFFE000u);
             pc[0][h] = a;
-            pc[1][h] = b * 0.00390625f;
-            pc[2][h] = (r - b) * 1.52587890625e-5f;
+            pc[1][h] = b * (kPlanes == 8 ? 256.f : 0.00390625f);
+            pc[2][h] = (r - b) * (kPlanes == 8 ? 65536.f : 1.52587890625e-5f);
             pc[3][h] = 0.f;
         }
 #pragma unroll
@@ -316,7 +340,8 @@ __device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t 
             for (int h = 0; h < 2; ++h) {
                 if constexpr (MC == 8) x.mn[nb][h] = pc[nb][h];
                 else if constexpr (MC == 4) x.mn[nb][h] = (g & 4) ? pc[2 * nb + 1][h] : pc[2 * nb][h];
-                else x.mn[nb][h] = (g & 4) ? ((g & 2) ? pc[3][h] : pc[2][h]) : ((g & 2) ? pc[1][h] : pc[0][h]);
+                else if constexpr (MC == 2) x.mn[nb][h] = (g & 4) ? ((g & 2) ? pc[3][h] : pc[2][h]) : ((g & 2) ? pc[1][h] : pc[0][h]);
+                else x.mn[nb][h] = g == 7 ? pc[0][h] : g == 6 ? pc[1][h] : g == 5 ? pc[2][h] : 0.f;
             }
     }
     // k-steps per pass through the scratch memory: [k-step][set][column][t] of 8 bytes, k-steps 32 bytes apart in banks
@@ -354,7 +379,7 @@ __device__ __forceinline__ bool mb_stage_x(const MbParams& p, int blk, uint32_t 
             for (int nb = 0; nb < NB; ++nb) x.b[ch * KC + jc][nb] = lds64(scratch + (uint32_t)jc * kStepBytes + (uint32_t)nb * 256u + 8u * (uint32_t)lane);
     }
     __syncwarp();
-    return finite;
+    return left;
 }
 
 template <int FMT, int MC, int NB>
@@ -366,7 +391,8 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 127u) & ~127u;
     __shared__ uint64_t bar_part[2];
-    __shared__ int abort_flag, nonfinite;
+    __shared__ int abort_flag;
+    __shared__ uint32_t left;  // activation rows for the plain loop
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int nw = p.nwk * p.rg, rgi = warp / p.nwk, wk = warp - rgi * p.nwk;
@@ -379,7 +405,7 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
 
     if (tid == 0) {
         abort_flag = 0;
-        nonfinite = 0;
+        left = 0;
         mbar_init(smem_u32(&bar_part[0]), nw);
         mbar_init(smem_u32(&bar_part[1]), nw);
         fence_mbar_init();
@@ -445,6 +471,12 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
                 for (int w = sub; w < p.nwk; w += p.tpo, at += (uint32_t)p.tpo * 512u) {
                     float c = __uint_as_float(lds32i<0>(at));
                     if constexpr (MC == 4) c = fmaf(256.f, __uint_as_float(lds32i<16>(at)), c);
+                    if constexpr (MC == 1) {
+                        const uint4 q = lds128i<0>(at), h = lds128i<16>(at);
+                        const uint32_t col[8] = {q.x, q.y, q.z, q.w, h.x, h.y, h.z, h.w};
+#pragma unroll
+                        for (int i = 1; i < 8; ++i) c = fmaf(c, 0.00390625f, __uint_as_float(col[i]));
+                    }
                     if constexpr (MC == 2) {
                         const float c1 = __uint_as_float(lds32i<8>(at)), c2 = __uint_as_float(lds32i<16>(at)), c3 = __uint_as_float(lds32i<24>(at));
                         c = fmaf(256.f, fmaf(256.f, fmaf(256.f, c3, c2), c1), c);
@@ -471,7 +503,8 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
         const int blk = ph * p.nwk + wk;
         if (it == 0 && blk < p.nblk) {
             // the slot of the tile before (at the start: the ring's last) is free until the next issue
-            if (!mb_stage_x<FMT, MC, NB>(p, blk, ring + (uint32_t)islot * kStage, lane, x)) nonfinite = 1;
+            const uint32_t rows = mb_stage_x<FMT, MC, NB>(p, blk, ring + (uint32_t)islot * kStage, lane, x);
+            if (rows && lane == 0) atomicOr(&left, rows);
         }
         issue();
         cp_async_wait<NS - 1>();
@@ -503,8 +536,7 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
         reduce(part + (uint32_t)(b * nw) * 512u);
     }
     __syncthreads();
-    if (nonfinite)
-        for (int m = 0; m < p.M; ++m) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, p.N, p.K, p.row_bytes, row_begin, n_rows);
+    if (left) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, 0, left, p.N, p.K, p.row_bytes, row_begin, n_rows);
 }
 
 // ---- host side ------------------------------------------------------------------------
@@ -568,10 +600,12 @@ static int launch_mb_f(MbParams& p, int sms, cudaStream_t st, bool* taken) {
     p.tpo = 1;
     while (p.tpo < 32 && p.tpo < p.nwk && 2 * p.tpo * n_out <= threads) p.tpo *= 2;
     *taken = true;
+    // One row of FP32: eight planes, whose cost is their staging (Q5_K 14336 x 4096 18.2 us, with four planes 18.1; 1024 x 4096 5.2, with four
+    // 4.4); four would send a token with one channel a thousand times the others to the plain loop. 16-bit values hardly need more than four.
+    if (p.M == 1 && p.x_dtype == B200Q_DT_F32) return launch_mb<FMT, 1, 1>(p, grid, smem, st);
     if (p.M <= 2) return launch_mb<FMT, 2, 1>(p, grid, smem, st);
     if (p.M <= 4) return launch_mb<FMT, 4, 2>(p, grid, smem, st);
-    if (p.x_dtype == B200Q_DT_F32) return launch_mb<FMT, 8, 4>(p, grid, smem, st);
-    return launch_mb<FMT, 8, 3>(p, grid, smem, st);
+    return launch_mb<FMT, 8, 4>(p, grid, smem, st);
 }
 
 // Launches the kernel when it takes the call (*taken = true): whole 256-element pieces, weights on a 16-byte

@@ -1,6 +1,6 @@
 // Pieces shared by the kernels that multiply raw quants on the warp-level tensor-core instructions (gemv_mb.cu: one to eight
 // activation rows on integer MMA; gemm_mm.cu: a few dozen on FP16 MMA): how a 256-element piece of a weight row lies in
-// shared memory, asynchronous 16-byte copies, activations as floats, and the plain FP32 loop for rows that are not finite.
+// shared memory, asynchronous 16-byte copies, activations as floats, and the plain FP32 loop for rows that they leave to it.
 #pragma once
 
 #include "common.cuh"
@@ -120,6 +120,25 @@ __device__ __forceinline__ void qm_to_f32(const uint4 (&r)[2], int x_dtype, floa
         }
     }
 }
+// Whether the bulk of some sub-block of 32 activations (f * s, eight per thread, four neighbouring threads) is lost in the error of its
+// representation: `err2` is the thread's sum of squared errors. More than half of the elements that are not zero must stand 2^21 above
+// the sub-block's root mean square of the error - so weights that are small in a few large channels leave a result with the
+// accuracy of FP32 products (3e-7), whatever those channels hold. The answer is the warp's.
+__device__ __forceinline__ bool qm_sub_block_lost(const float (&f)[8], float s, float err2) {
+    err2 += __shfl_xor_sync(0xffffffffu, err2, 1);
+    err2 += __shfl_xor_sync(0xffffffffu, err2, 2);
+    const float limit = err2 * 137438953472.0f;  // 2^42 / 32
+    int count = 0;  // twice the elements below the limit, less those that are not zero
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float v = f[k] * s;
+        count += (v * v < limit ? 2 : 0) - 1;
+        count += v == 0.f ? (limit > 0.f ? -1 : 1) : 0;
+    }
+    count += __shfl_xor_sync(0xffffffffu, count, 1);
+    count += __shfl_xor_sync(0xffffffffu, count, 2);
+    return __any_sync(0xffffffffu, count > 0);
+}
 __device__ __forceinline__ float qm_bias(const void* bias, int dtype, int n) {
     if (!bias) return 0.f;
     if (dtype == B200Q_DT_F32) return static_cast<const float*>(bias)[n];
@@ -132,27 +151,37 @@ __device__ __forceinline__ void qm_store(void* Y, int dtype, size_t at, float v)
     else static_cast<__nv_bfloat16*>(Y)[at] = __float2bfloat16_rn(v);
 }
 
-// Y of weight rows [row_begin, row_begin + n_rows) and activation row m in FP32 from memory, a warp per row: for activations
-// that are not finite, where a result is what IEEE arithmetic makes of infinities and NaN.
+// Y of weight rows [row_begin, row_begin + n_rows) and the activation rows m0 + i of the bits i of `rows`, in FP32 from memory, a
+// warp per weight row: for activations that are not finite, where a result is what IEEE arithmetic makes of infinities and NaN, and for
+// ones whose range the fixed-point forms do not hold.
 template <int FMT>
-__device__ __forceinline__ void qm_plain_rows(const uint8_t* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int m, int N,
-                                              int K, int row_bytes, int row_begin, int n_rows) {
+__device__ __noinline__ void qm_plain_rows(const uint8_t* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int m0, uint32_t rows,
+                                              int N, int K, int row_bytes, int row_begin, int n_rows) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int r = warp; r < n_rows; r += nw) {
         const int n = row_begin + r;
-        float acc = 0.f;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int u = lane; u < (K >> 3); u += 32) {
-            float w[8], v[8];
-            uint4 raw[2];
+            float w[8];
             decode8<FMT, LdDep>(W + (size_t)n * row_bytes, u, w);
-            qm_load_raw(X, x_dtype == B200Q_DT_F32, K, m, 8 * u, raw);
-            qm_to_f32(raw, x_dtype, v);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc = fmaf(w[k], v[k], acc);
+            for (int i = 0; i < 8; ++i)
+                if (rows >> i & 1u) {
+                    float v[8];
+                    uint4 raw[2];
+                    qm_load_raw(X, x_dtype == B200Q_DT_F32, K, m0 + i, 8 * u, raw);
+                    qm_to_f32(raw, x_dtype, v);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[i] = fmaf(w[k], v[k], acc[i]);
+                }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) qm_store(Y, y_dtype, (size_t)m * N + n, acc + qm_bias(bias, x_dtype, n));
+        for (int i = 0; i < 8; ++i)
+            if (rows >> i & 1u) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+                if (lane == 0) qm_store(Y, y_dtype, (size_t)(m0 + i) * N + n, acc[i] + qm_bias(bias, x_dtype, n));
+            }
     }
 }
 

@@ -146,6 +146,46 @@ def test_activations_that_are_not_finite(fmt, ops_raw):
             assert torch.allclose(y[ok], want[ok], rtol=1e-4, atol=1e-4)
 
 
+def _wide_operands(fmt, N, K, M, dtype, base=10.0):
+    """Weights that are zero in one channel of every 256 and activations that are base^m times the others there (row m): the channel adds nothing to a
+    result, but it sets the scale of whatever represents the 256 together."""
+    blocks = synth.make_blocks(fmt, N, K, seed=N).reshape(-1, synth.BLOCK_BYTES[fmt])
+    if fmt == synth.Q4_0:  # element 5 of every eighth block: nibble 8
+        z = blocks.reshape(N, -1, 18)[:, ::8]
+        z[..., 2 + 5] = (z[..., 2 + 5] & 0xF0) | 8
+    elif fmt == synth.Q6_K:  # 6-bit value 32
+        blocks[:, 5] &= 0xF0
+        blocks[:, 128 + 5] = (blocks[:, 128 + 5] & 0xFC) | 2
+    else:  # Q5_K: q = 0 and no min in the first sub-block
+        blocks[:, 8] &= 0xC0
+        blocks[:, 16 + 5] &= 0xFE
+        blocks[:, 48 + 5] &= 0xF0
+    x = synth.make_activations(M, K, seed=K)
+    x[:, 5::256] *= (base ** np.arange(M, dtype=np.float64)[:, None]).astype(np.float32)
+    x = torch.from_numpy(x).to(DT[dtype])
+    assert torch.isfinite(x).all()
+    want = oracle.cpu().matmul(fmt, blocks.reshape(-1), x.float().numpy(), threads=8, want_f64=True)[1]
+    return torch.from_numpy(blocks.reshape(-1).copy()).cuda(), x.cuda(), want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", [synth.Q5_K, synth.Q6_K, synth.Q4_0])
+def test_a_channel_far_above_the_others(fmt, ops_raw):
+    """What a channel without weight costs the rest of its block: nothing, in FP32 as in the 16-bit types."""
+    ops = ops_raw
+    N, K = 90, 2304
+    for M, dtype, base in ((8, "f32", 10), (8, "bf16", 10), (6, "f16", 6), (4, "f32", 100), (2, "f32", 1000), (2, "f32", 1e5)):
+        W, x, want = _wide_operands(fmt, N, K, M, dtype, base)
+        ops.set_option("gemv_hm", 0)
+        ops.set_option("gemv_mb", 2)
+        rows = ops.gemv(fmt, W, x, N, out_dtype=torch.float32)
+        assert _last_kernel() == MB
+        each = torch.cat([ops.gemv(fmt, W, x[m:m + 1], N, out_dtype=torch.float32) for m in range(M)])
+        for m in range(M):
+            for y in (rows, each):
+                assert oracle.rel_l2(y[m].cpu().numpy(), want[m]) < 2e-6, (M, dtype, m)
+
+
 @pytest.mark.gpu
 def test_magnitudes_that_fp16_cannot_hold(ops_raw):
     """FP32 and BF16 activations far outside FP16's range are scaled, not rounded away."""
@@ -153,9 +193,9 @@ def test_magnitudes_that_fp16_cannot_hold(ops_raw):
     fmt, N, K = synth.Q5_K, 96, 2048
     Wh = synth.make_blocks(fmt, N, K, seed=8)
     W = torch.from_numpy(Wh).cuda()
-    for M in (2, 6, 24):
+    for M in (1, 2, 6, 24):
         for dtype in ("f32", "bf16"):
-            for scale in (1e-25, 1e-6, 1e6, 1e25):
+            for scale in (1e-30, 1e-25, 1e-6, 1e6, 1e25, 1e30):
                 x = (torch.from_numpy(synth.make_activations(M, K, seed=9)) * scale).to(DT[dtype])
                 want = oracle.cpu().matmul(fmt, Wh, x.float().numpy(), threads=8, want_f64=True)[1]
                 y = ops.linear(fmt, W, x.cuda(), N, out_dtype=torch.float32).cpu().numpy()
