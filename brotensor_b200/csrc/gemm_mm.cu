@@ -6,8 +6,10 @@
 //   * A fragments are the quants as FP16 integers: masked into the mantissas of two halves that hold 1024 (one logic operation), from
 //     which a packed subtraction takes the 1024 (and Q4_0's offset of 8) off, exactly. (Left as subnormals, q * 2^-24, they would save
 //     the subtraction, but the tensor cores align products without normalising them first: 1e-6 against 1.2e-7 of error.)
-//   * B fragments are the activations in FP16, scaled per token by a power of two to [2^14, 2^15): FP16 inputs are exact,
-//     FP32 inputs are split into two FP16 terms (22 bits), each multiplied.
+//   * B fragments are the activations in FP16, scaled per token by a power of two to [2^14, 2^15) (FP16 inputs never down): FP16 inputs
+//     are exact, BF16 ones down to 2^-31 of the token's largest, and FP32 inputs are split into two FP16 terms, each multiplied, that hold
+//     them to 2^-22 of their own size down to 2^-17 of the largest. Where that range is not enough for the bulk of some sub-block
+//     (qm_sub_block_lost, and likewise the sums below), the token is marked for the plain FP32 loop, as are infinities and NaN.
 //   * Every sub-block's products are summed on the tensor cores in FP32 and then multiplied by its scale in FP32 (four
 //     FMA per 16 x 8 x 32 products). The minimums' term of Q5_K is one more MMA per 256 k: A the 6-bit mins, B the sub-block
 //     sums of the activations as two FP16 terms.
@@ -31,14 +33,14 @@ constexpr int kMmMaxTiles = 8;    // 16-row tiles of a CTA at a time
 
 struct MmParams {
     const uint8_t* W;
-    const void* X;     // the caller's activations (only read for tokens that are not finite)
+    const void* X;     // the caller's activations (only read for the marked tokens)
     const void* bias;
     void* Y;           // first token row of this pass
     // prepared activations, this pass's first token: [K/256][tok_stride] rows of 512 bytes (high and, FP32 only, low terms) and of
-    // 32 bytes (sub-block sums), 2^-e per token, and a mark per token that is not finite
+    // 32 bytes (sub-block sums), 2^-e per token, and a mark per token that goes to the plain loop
     const uint8_t *Xh, *Xl, *Xs;
     const float* inv;
-    const int* nonfinite;
+    const int* plain;
     int tokens, tok_stride, N, K;
     int x_dtype, y_dtype;
     int row_bytes, nblk;
@@ -51,7 +53,7 @@ struct MmParams {
 // One block per token. pair8: a thread of the GEMM holds elements 8t .. 8t+7 of a sub-block (Q4_K, Q5_K), else 4t .. 4t+3 and
 // 16+4t .. 16+4t+3. Register i of its four per row multiplies two of them: image position 8 i + 2 t + j of the sub-block.
 __global__ void __launch_bounds__(256) gemm_mm_prep_kernel(const void* X, int x_dtype, int K, int tok_stride, int pair8, uint8_t* Xh,
-                                                           uint8_t* Xl, uint8_t* Xs, float* inv, int* nonfinite) {
+                                                           uint8_t* Xl, uint8_t* Xs, float* inv, int* plain) {
     __shared__ uint32_t warp_top[8];
     const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const bool f32 = x_dtype == B200Q_DT_F32;
@@ -73,12 +75,10 @@ __global__ void __launch_bounds__(256) gemm_mm_prep_kernel(const void* X, int x_
     for (int w = 0; w < 8; ++w) top = max(top, warp_top[w]);
     const bool finite = top < 0x7F800000u;
     int e = 14 + 127 - (int)(top >> 23);
-    e = (top == 0 || !finite) ? 0 : max(-126, min(126, e));
+    bool lost = !finite || (top != 0 && e > 126);  // (below 2^-112 the scale ends)
+    e = (top == 0 || !finite) ? 0 : max(x_dtype == B200Q_DT_F16 ? 0 : -126, min(126, e));
     const float s = __uint_as_float((uint32_t)(e + 127) << 23);
-    if (tid == 0) {
-        inv[m] = __uint_as_float((uint32_t)(127 - e) << 23);
-        nonfinite[m] = finite ? 0 : 1;
-    }
+    if (tid == 0) inv[m] = __uint_as_float((uint32_t)(127 - e) << 23);
     for (int c = tid; c < (K >> 3); c += 256) {  // K % 256 == 0: whole warps are in or out
         uint4 raw[2];
         float f[8];
@@ -87,13 +87,26 @@ __global__ void __launch_bounds__(256) gemm_mm_prep_kernel(const void* X, int x_
         const int blk = c >> 5, sub = (c >> 2) & 7, t = c & 3;
         const size_t row = (size_t)blk * tok_stride + m;
         float sum = 0.f;
+        uint32_t mine = 0;
         __half h[8], l[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const float v = f[k] * s;
             sum += v;
+            mine = max(mine, __float_as_uint(f[k]) & 0x7FFFFFFFu);
             h[k] = __float2half_rn(v);
             l[k] = __float2half_rn(v - __half2float(h[k]));
+        }
+        // Where every eight neighbours reach 2^-12 of the token's largest, the terms hold enough of them; elsewhere it is looked at closely.
+        const bool uneven = __any_sync(0xffffffffu, mine + (12u << 23) < top);
+        if (uneven) {
+            float err2 = 0.f;  // where the subnormals cut bits off
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float v = f[k] * s, err = kErrUp * (v - __half2float(h[k]) - (f32 ? __half2float(l[k]) : 0.f));
+                if (fabsf(v) < 0.125f) err2 = fmaf(err, err, err2);
+            }
+            lost |= qm_sub_block_lost(f, s, err2);
         }
         auto put = [&](uint8_t* img, const __half(&v)[8]) {
             uint8_t* base = img + row * 512;
@@ -116,15 +129,25 @@ __global__ void __launch_bounds__(256) gemm_mm_prep_kernel(const void* X, int x_
         if (pair8) {  // sub-block sums / 64 as two FP16 terms: [t2][high 2 t2, 2 t2 + 1, low 2 t2, 2 t2 + 1]
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum *= 0.015625f;
+            const __half a = __float2half_rn(sum), b = __float2half_rn(sum - __half2float(a));
             if (t == 0) {
-                sum *= 0.015625f;
-                const __half a = __float2half_rn(sum);
                 __half* d = reinterpret_cast<__half*>(Xs + row * 32) + 4 * (sub >> 1) + (sub & 1);
                 d[0] = a;
-                d[2] = __float2half_rn(sum - __half2float(a));
+                d[2] = b;
+            }
+            if (uneven) {
+                float size = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) size += fabsf(f[k] * s);
+                size += __shfl_xor_sync(0xffffffffu, size, 1);
+                size += __shfl_xor_sync(0xffffffffu, size, 2);
+                lost |= fabsf(sum - __half2float(a) - __half2float(b)) * 2097152.0f > size * 0.015625f;
             }
         }
     }
+    lost = __syncthreads_or(lost) != 0;
+    if (tid == 0) plain[m] = lost ? 1 : 0;
 }
 
 // ---- the GEMM -------------------------------------------------------------------------------------------
@@ -351,13 +374,13 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
             for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
         ++it;
     }
-    // Tokens that are not finite: their results in FP32 arithmetic, which knows infinities and NaN.
+    // The marked tokens: their results in FP32 arithmetic.
     bool any = false;
-    for (int m = lane; m < p.tokens; m += 32) any |= p.nonfinite[m] != 0;
+    for (int m = lane; m < p.tokens; m += 32) any |= p.plain[m] != 0;
     if (__any_sync(0xffffffffu, any)) {
         __syncthreads();  // the stores above come first
         for (int m = 0; m < p.tokens; ++m)
-            if (p.nonfinite[m]) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, 1u, p.N, p.K, p.row_bytes, row_begin, n_rows);
+            if (p.plain[m]) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, 1u, p.N, p.K, p.row_bytes, row_begin, n_rows);
     }
 }
 
@@ -447,7 +470,7 @@ int launch_gemm_mm(int fmt, const void* W, const void* X, int x_dtype, const voi
     uint8_t* xl = xh + mm_image_bytes(M, K);
     uint8_t* xs = xl + (x_dtype == B200Q_DT_F32 ? mm_image_bytes(M, K) : 0);
     float* inv = reinterpret_cast<float*>(xs + mm_sums_bytes(M, K));
-    int* nonfinite = reinterpret_cast<int*>(inv + stride);
+    int* plain = reinterpret_cast<int*>(inv + stride);
     const int passes = (M + kMmMaxTokens - 1) / kMmMaxTokens, per = ((M + passes - 1) / passes + 7) & ~7;
     bool prepared = false;
     for (int t0 = 0; t0 < M; t0 += per) {
@@ -460,7 +483,7 @@ int launch_gemm_mm(int fmt, const void* W, const void* X, int x_dtype, const voi
         p.Xl = xl + (size_t)t0 * 512;
         p.Xs = xs + (size_t)t0 * 32;
         p.inv = inv + t0;
-        p.nonfinite = nonfinite + t0;
+        p.plain = plain + t0;
         p.tokens = M - t0 < per ? M - t0 : per;
         p.tok_stride = stride;
         p.N = N;
@@ -471,7 +494,7 @@ int launch_gemm_mm(int fmt, const void* W, const void* X, int x_dtype, const voi
         if (!prepared) {
             prepared = true;
             B200Q_CUDA_TRY(launch_dep(pdl_option() >= 0, gemm_mm_prep_kernel, dim3((unsigned)M), dim3(256), 0, st, X, x_dtype, K, stride,
-                                      (int)(fmt == kQ5_K), xh, xl, xs, inv, nonfinite));
+                                      (int)(fmt == kQ5_K), xh, xl, xs, inv, plain));
         }
         bool ok = false;
         int rc = B200Q_OK;

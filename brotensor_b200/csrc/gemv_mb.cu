@@ -292,7 +292,7 @@ __device__ __forceinline__ uint32_t mb_stage_x(const MbParams& p, int blk, uint3
                     float err2 = 0.f;  // of eight planes at most 2^-32 each
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        const float err = kPlanes == 8 ? 2.3283064365386963e-10f : f[k] * s - (float)__float2int_rn(f[k] * s);
+                        const float err = kErrUp * (kPlanes == 8 ? 2.3283064365386963e-10f : f[k] * s - (float)__float2int_rn(f[k] * s));
                         err2 = fmaf(err, err, err2);
                     }
                     if (qm_sub_block_lost(f, s, err2)) left |= 1u << m;

@@ -121,19 +121,20 @@ __device__ __forceinline__ void qm_to_f32(const uint4 (&r)[2], int x_dtype, floa
     }
 }
 // Whether the bulk of some sub-block of 32 activations (f * s, eight per thread, four neighbouring threads) is lost in the error of its
-// representation: `err2` is the thread's sum of squared errors. More than half of the elements that are not zero must stand 2^21 above
-// the sub-block's root mean square of the error - so weights that are small in a few large channels leave a result with the
-// accuracy of FP32 products (3e-7), whatever those channels hold. The answer is the warp's.
+// representation: `err2` is the thread's sum of squared errors, each times kErrUp (squares of what is left of activations 2^90 below the
+// largest are subnormal). At least half of the elements that are not zero must stand 2^21 above the sub-block's root mean square
+// of the error - so weights that are small in a few large channels leave a result with the accuracy of FP32 products (3e-7),
+// whatever those channels hold. The answer is the warp's.
+constexpr float kErrUp = 1073741824.0f;  // 2^30
 __device__ __forceinline__ bool qm_sub_block_lost(const float (&f)[8], float s, float err2) {
     err2 += __shfl_xor_sync(0xffffffffu, err2, 1);
     err2 += __shfl_xor_sync(0xffffffffu, err2, 2);
     const float limit = err2 * 137438953472.0f;  // 2^42 / 32
-    int count = 0;  // twice the elements below the limit, less those that are not zero
+    int count = 0;                               // elements below the limit, less those above
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const float v = f[k] * s;
-        count += (v * v < limit ? 2 : 0) - 1;
-        count += v == 0.f ? (limit > 0.f ? -1 : 1) : 0;
+        const float v = f[k] * s * kErrUp;
+        count += f[k] == 0.f ? 0 : v * v <= limit ? 1 : -1;
     }
     count += __shfl_xor_sync(0xffffffffu, count, 1);
     count += __shfl_xor_sync(0xffffffffu, count, 2);

@@ -187,6 +187,27 @@ def test_a_channel_far_above_the_others(fmt, ops_raw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fmt", [synth.Q5_K, synth.Q4_0])
+def test_a_channel_far_above_the_others_in_a_prompt(fmt, ops_raw):
+    ops = ops_raw
+    N, K = 90, 2304
+    for M, dtype, base in ((20, "f32", 10), (20, "bf16", 30), (17, "f32", 30), (12, "f16", 2.2)):
+        W, x, want = _wide_operands(fmt, N, K, M, dtype, base)
+        ops.set_option("gemv_hm", 0)  # (up to sixteen rows of 16-bit activations are its)
+        y = ops.linear(fmt, W, x, N, out_dtype=torch.float32).cpu().numpy()
+        assert _last_kernel() == MM
+        for m in range(M):
+            assert oracle.rel_l2(y[m], want[m]) < 2e-6, (M, dtype, m)
+    # the other end: a token whose largest value is near FP16's, and one far below FP32's normal scale
+    Wh = synth.make_blocks(fmt, N, K, seed=2)
+    for dtype, scale in (("f16", 12000.0), ("f32", 1e-35)):
+        x = (torch.from_numpy(synth.make_activations(24, K, seed=9)) * scale).to(DT[dtype])
+        want = oracle.cpu().matmul(fmt, Wh, x.float().numpy(), threads=8, want_f64=True)[1]
+        y = ops.linear(fmt, torch.from_numpy(Wh).cuda(), x.cuda(), N, out_dtype=torch.float32).cpu().numpy()
+        assert oracle.rel_l2(y / np.float32(scale), want / scale) < 2e-6
+
+
+@pytest.mark.gpu
 def test_magnitudes_that_fp16_cannot_hold(ops_raw):
     """FP32 and BF16 activations far outside FP16's range are scaled, not rounded away."""
     ops = ops_raw
