@@ -206,12 +206,14 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 127u) & ~127u;
     const uint8_t* smem = smem_raw + (sbase - smem_u32(smem_raw));
+    __shared__ uint32_t plain[kMmMaxTokens / 32];  // bits of the tokens for the plain loop
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int nthreads = 32 * p.mt * KG;
     const int ki = warp / p.mt, mi = warp - ki * p.mt;
     const int cta = (int)blockIdx.x;
     const int row_begin = cta * p.row_q + min(cta, p.row_r), n_rows = p.row_q + (cta < p.row_r ? 1 : 0);
     const int rows_it = kQmTile * p.mt, iters = (n_rows + rows_it - 1) / rows_it, steps = iters * p.nblk;
+    if (tid < kMmMaxTokens / 32) plain[tid] = 0;
     grid_dep_launch();
 
     // Next stage to fetch: rows of iteration ii, block ib, into ring slot islot.
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
     const int s_first = ki * kSubs;
     const uint32_t b_lane = (uint32_t)((lane & 7) * 512);
     int slot = 0, it = 0, blk = 0;
+    float odd = 0.f;  // not zero once one of the thread's results is not finite (an infinite scale)
     for (int step = 0; step < steps; ++step) {
         if (p.n_stages == 4) cp_async_wait<2>();
         else if (p.n_stages == 3) cp_async_wait<1>();
@@ -362,6 +365,7 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
                         for (int j = 0; j < 2; ++j) {
                             const int m = 8 * n + 2 * t + j;
                             if (m < p.tokens) {
+                                odd = fmaf(acc[n][2 * h + j], 0.f, odd);
                                 qm_store(p.Y, p.y_dtype, (size_t)m * p.N + row, fmaf(acc[n][2 * h + j], p.inv[m], bv));
                             }
                         }
@@ -374,14 +378,13 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
             for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
         ++it;
     }
-    // The marked tokens: their results in FP32 arithmetic.
-    bool any = false;
-    for (int m = lane; m < p.tokens; m += 32) any |= p.plain[m] != 0;
-    if (__any_sync(0xffffffffu, any)) {
-        __syncthreads();  // the stores above come first
-        for (int m = 0; m < p.tokens; ++m)
-            if (p.plain[m]) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, 1u, p.N, p.K, p.row_bytes, row_begin, n_rows);
-    }
+    // The marked tokens, and all of them where a result is not finite: their results in FP32 arithmetic.
+    if (!(odd == 0.f)) atomicOr(&plain[0], ~0u), atomicOr(&plain[1], ~0u);
+    if (tid < p.tokens && p.plain[tid]) atomicOr(&plain[tid >> 5], 1u << (tid & 31));
+    __syncthreads();  // (and the stores above come first)
+    for (int m = 0; m < p.tokens; m += 8)
+        if (const uint32_t rows = plain[m >> 5] >> (m & 31) & 0xFFu & ((1u << min(8, p.tokens - m)) - 1u))
+            qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, m, rows, p.N, p.K, p.row_bytes, row_begin, n_rows);
 }
 
 // ---- host side ------------------------------------------------------------------------------------------

@@ -28,7 +28,8 @@
 // Measured (one row, us, plain-load kernel -> this one): Q5_K 14336 x 4096 39.8 -> 17.1, 4096 x 4096 16.9 -> 7.4, 4096 x 14336 50.6 -> 19.5; Q4_0 29.5 -> 17.6,
 // 13.1 -> 7.1, 40.4 -> 19.4; Q6_K 2560 x 6912 20.8 -> 12.4. It runs at half of the memory's rate for one row: 58 instructions per k-step of
 // 16 x 32, of which the kernel's own work is about 25 and the rest is waiting for the others at a tile's end.
-// Rows of activations that are not finite or not held take a plain FP32 loop at the end of the launch (qm_plain_rows).
+// Rows of activations that are not finite or not held, and all rows where a result is not finite, take a plain FP32 loop at the end of the
+// launch (qm_plain_rows): an integer sum of zero times an infinite scale is not what the decoded weights give.
 //
 // Takes the place of brotensor's decode GEMVs (src/cuda/q4k.cu:159-224, q6k.cu:117-176, q8_0.cu:75-138) and of the
 // per-row loop of its batched ops for small B (q4k.cu:413-418).
@@ -456,6 +457,7 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
     const int tpo_log = 31 - __clz(p.tpo), sub = tid & (p.tpo - 1), per_pass = (nw * 32) >> tpo_log, n_out = kQmTile * p.rg * p.M;
     const int o_first = tid >> tpo_log, o_gm = o_first >> 4;
     const int g_first = o_gm / p.M, m_first = o_gm - g_first * p.M;
+    float odd = 0.f;  // not zero once one of the thread's results is not finite: an infinite scale, or more than FP32 holds on the way
     auto reduce = [&](uint32_t buf) {
         int gr = g_first, m = m_first;
         for (int base = 0; base < n_out; base += per_pass) {
@@ -490,7 +492,10 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
                 const uint32_t ya = yacc + (uint32_t)(r * p.M + m) * 4u;
                 if (rp > 0) s += __uint_as_float(lds32i<0>(ya));
                 if (rp + 1 < p.phases) sts32(ya, __float_as_uint(s));  // read by this thread alone
-                else qm_store(p.Y, p.y_dtype, (size_t)m * p.N + row_begin + r, s + qm_bias(p.bias, p.x_dtype, row_begin + r));
+                else {
+                    odd = fmaf(s, 0.f, odd);
+                    qm_store(p.Y, p.y_dtype, (size_t)m * p.N + row_begin + r, s + qm_bias(p.bias, p.x_dtype, row_begin + r));
+                }
             }
         }
         if (++ri == iters) { ri = 0; ++rp; }
@@ -535,6 +540,7 @@ __global__ void __launch_bounds__(kMbMaxWarps * 32, 1) gemv_mb_kernel(const __gr
         __syncwarp();
         reduce(part + (uint32_t)(b * nw) * 512u);
     }
+    if (!(odd == 0.f)) atomicOr(&left, (1u << p.M) - 1u);
     __syncthreads();
     if (left) qm_plain_rows<FMT>(p.W, p.X, p.x_dtype, p.bias, p.Y, p.y_dtype, 0, left, p.N, p.K, p.row_bytes, row_begin, n_rows);
 }

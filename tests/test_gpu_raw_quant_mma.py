@@ -146,6 +146,38 @@ def test_activations_that_are_not_finite(fmt, ops_raw):
             assert torch.allclose(y[ok], want[ok], rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", FMTS)
+def test_scales_that_are_not_finite(fmt, ops_raw):
+    """A block whose FP16 scale is infinite gives what FP32 arithmetic on the decoded weights gives, also where its quants sum up to nothing."""
+    ops = ops_raw
+    N, K = 200, 1280
+    at = 208 if fmt == synth.Q6_K else 0
+    blocks = synth.make_blocks(fmt, N, K, seed=3).reshape(-1, synth.BLOCK_BYTES[fmt])
+    per_row = blocks.shape[0] // N
+    for row, bits in ((3, 0x7C00), (77, 0xFC00), (130, 0x7E00)):
+        blocks[row * per_row + 1, at:at + 2] = (bits & 255, bits >> 8)
+    W = torch.from_numpy(blocks.reshape(-1).copy()).cuda()
+    for M, dtype in ((1, "f32"), (1, "f16"), (3, "f16"), (3, "f32"), (7, "f32"), (20, "f16"), (20, "f32")):
+        if fmt not in (synth.Q5_K, synth.Q4_0) and (M > 8 or (dtype == "f32" and fmt != synth.Q6_K)):
+            continue  # (formats and types with other kernels)
+        x = torch.from_numpy(synth.make_activations(M, K, seed=4)).to(DT[dtype]).cuda()
+        x[0] = 0
+        for hm in (1, 2, 0):
+            if fmt in (synth.Q4_K, synth.Q8_0) and hm != 2:
+                continue
+            ops.set_option("gemv_hm", hm)
+            y = ops.linear(fmt, W, x, N, out_dtype=torch.float32)
+            assert _last_kernel() in (HM, MB, MM)
+            ops.set_option("gemv_path", 1)
+            want = torch.cat([ops.gemv(fmt, W, x[i:i + 1], N, out_dtype=torch.float32) for i in range(M)])
+            ops.set_option("gemv_path", 0)
+            assert not torch.isfinite(want).all()
+            assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(y[torch.isinf(y)], want[torch.isinf(want)])
+            ok = torch.isfinite(want)
+            assert torch.allclose(y[ok], want[ok], rtol=1e-4, atol=1e-4)
+
+
 def _wide_operands(fmt, N, K, M, dtype, base=10.0):
     """Weights that are zero in one channel of every 256 and activations that are base^m times the others there (row m): the channel adds nothing to a
     result, but it sets the scale of whatever represents the 256 together."""
