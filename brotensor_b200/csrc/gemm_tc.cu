@@ -213,9 +213,9 @@ static bool gemm_tc_takes(int fmt, const void* W, int M, int K) {
     return fmt == kQ4_K || fmt == kQ6_K || fmt == kQ8_0;
 }
 
-// How a call is cut into work for the 74 CTA pairs of the chip: passes of up to 512 tokens (each decodes the weights
-// again), and K splits (equal shares, whole 256-element blocks, at least eight k-blocks each; the partial sums go through the
-// workspace and are added in a fixed order by a second kernel). One launch holds all of it, so the plan is the one whose waves
+// How a call is cut into work for the 74 CTA pairs of the chip (148 SMs, the only part sm_100a names): passes of up to 512 tokens (each
+// decodes the weights again), and K splits (equal shares, whole 256-element blocks, at least eight k-blocks each; the partial sums go
+// through the workspace and are added in a fixed order by a second kernel). One launch holds all of it, so the plan is the one whose waves
 // take least by this model (us, fitted to B200): a 64-k stage costs the larger of its MMAs (0.85 for 512 tokens) and its
 // decode; a tile adds its start and epilogue; split sums are written and read once. Passes launched one after the other
 // left most pairs idle - 2000 tokens of 4096 rows were four launches of 16 tiles, split in four - and 400 tokens a pass
@@ -226,18 +226,19 @@ int gemm_get_split() { return g_gemm_split; }
 struct GemmPlan {
     int tok_pass, split;
 };
-static GemmPlan gemm_plan(int fmt, int M, int N, int K, bool may_split) {
+// The best plan of a split from s_min to s_max.
+static GemmPlan gemm_plan(int fmt, int M, int N, int K, int s_min, int s_max) {
     const int pairs = ((N + kGemmRows - 1) / kGemmRows + 1) / 2, n_kb = K / kBK, chip = 74;
     const double decode = (fmt == kQ6_K || fmt == kQ6_KP) ? 1.05 : fmt == kQ8_0 ? 0.75 : 0.69;
-    const int p_min = (M + kMaxTokens - 1) / kMaxTokens;
+    const int p_min = (M + kMaxTokens - 1) / kMaxTokens, p_max = p_min < 6 ? 2 * p_min + 2 : p_min + 8;
     GemmPlan best = {kMaxTokens, 1};
     double best_t = -1;
-    for (int p = p_min; p <= 2 * p_min + 2; ++p) {
+    for (int p = p_min; p <= p_max; ++p) {
         const int pass = p == 1 ? round_up16(M) : ((M + p - 1) / p + 31) & ~31, passes = (M + pass - 1) / pass;
         if (p > p_min && pass < 128) break;
-        for (int s = 1; s <= 8; ++s) {
-            if (s > 1 && (!may_split || !g_gemm_split || N % 4 != 0 || n_kb % (4 * s) != 0 || n_kb / s < 8)) continue;
-            const int waves = (pairs * passes * s + chip - 1) / chip;
+        for (int s = s_min; s <= s_max; ++s) {
+            if (s > 1 && (n_kb % (4 * s) != 0 || n_kb / s < 8)) continue;
+            const long long waves = ((long long)pairs * passes * s + chip - 1) / chip;
             const double stage = 0.85 * pass / 512 > decode ? 0.85 * pass / 512 : decode;
             double t = waves * ((double)n_kb / s * stage + 3.0 + 4.0 * pass / 512);
             if (s > 1) t += 2.5 + (double)s * M * N * 8 / 5.0e6;
@@ -248,6 +249,31 @@ static GemmPlan gemm_plan(int fmt, int M, int N, int K, bool may_split) {
         }
     }
     return best;
+}
+// The split is chosen for M rounded up to a sixteenth to an eighth of itself (at least 32 tokens), so that the workspace of a call can
+// cover those of all shorter ones by looking at a few sizes (gemm_split_floats).
+static int gemm_split_unit(int M) {
+    int unit = 32;
+    while (M > 16 * (long long)unit) unit *= 2;
+    return unit;
+}
+static int gemm_split(int fmt, int M, int N, int K) {
+    if (!g_gemm_split || g_gemm_pair == 0 || N % 4 != 0) return 1;
+    const int unit = gemm_split_unit(M);
+    return M > (1 << 24) ? 1 : gemm_plan(fmt, (M + unit - 1) / unit * unit, N, K, 1, 8).split;
+}
+// Room for the partial sums of M tokens or fewer: a workspace made for the longest prompt does for every shorter one. Whole splits of
+// min(M, 512) tokens.
+static size_t gemm_split_floats(int fmt, int M, int N, int K) {
+    const size_t rows = M < kMaxTokens ? M : kMaxTokens;
+    size_t splits = 0;
+    for (int m = 0; m < M && m < (1 << 24);) {
+        m += gemm_split_unit(m + 1);
+        const int s = gemm_split(fmt, m, N, K);
+        const size_t own = m <= kMaxTokens ? s : ((size_t)s * (m < M ? m : M) + kMaxTokens - 1) / kMaxTokens;
+        if (s > 1 && own > splits) splits = own;
+    }
+    return splits * rows * N;
 }
 static size_t gemm_xp_bytes(int M, int K) { return ((size_t)(K / kBK) * (size_t)round_up16(M) * 128u + 255u) & ~(size_t)255u; }
 
@@ -261,9 +287,7 @@ size_t gemm_tc_workspace_min_bytes(int fmt, int x_dtype, int M, int N, int K) {
 size_t gemm_tc_workspace_bytes(int fmt, int x_dtype, int M, int N, int K) {
     (void)x_dtype;
     if (!gemm_tc_takes(fmt, nullptr, M, K)) return 0;
-    const int s = gemm_plan(fmt, M, N, K, g_gemm_pair != 0).split;
-    const size_t rows = M <= kMaxTokens ? M : (size_t)((M + kMaxTokens - 1) / kMaxTokens) * kMaxTokens;
-    return gemm_xp_bytes(M, K) + (s > 1 ? s * rows * N * sizeof(float) : 0);
+    return gemm_xp_bytes(M, K) + gemm_split_floats(fmt, M, N, K) * sizeof(float);
 }
 
 template <int FMT>
@@ -291,7 +315,10 @@ int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const voi
     // (the reduction kernel moves four neighbouring outputs at a time: Y and an FP32 bias must be aligned for that)
     const bool quads_ok = (reinterpret_cast<uintptr_t>(Y) & (y_dtype == B200Q_DT_F32 ? 15 : 3)) == 0 &&
                           (!bias || x_dtype != B200Q_DT_F32 || (reinterpret_cast<uintptr_t>(bias) & 15) == 0);
-    const GemmPlan plan = gemm_plan(fmt, M, N, K, g_gemm_pair != 0 && ws && quads_ok && ws_bytes >= gemm_tc_workspace_bytes(fmt, x_dtype, M, N, K));
+    // Split wherever the call's own partial sums fit behind the image, so that the bits do not depend on how much larger the workspace is.
+    int split = ws && quads_ok ? gemm_split(fmt, M, N, K) : 1;
+    if (split > 1 && ws_bytes < need + (size_t)split * M * N * sizeof(float)) split = 1;
+    const GemmPlan plan = gemm_plan(fmt, M, N, K, split, split);
     if (!ws || ws_bytes < need) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
     if (reinterpret_cast<uintptr_t>(ws) & 255) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace must be 256-byte aligned");
     const int tok_total = round_up16(M);

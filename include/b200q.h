@@ -211,11 +211,14 @@ int b200q_gemv_shard_topk(int fmt, const void* W_shard, const void* x, int x_dty
  *   Y(M,N) = X(M,K) * decode(W(N,K))^T (+ bias(N)),   FP16 operands, FP32 accumulation.
  * `ws` is caller-owned scratch of at least b200q_gemm_workspace_bytes() bytes,
  * 256-byte aligned (it holds the activations converted to the operand layout
- * and, for matrices of few rows, whose k range is split over several CTA
- * pairs, the FP32 partial sums: splits x M x N floats, M above 512
- * rounded up to a multiple of it);
- * it may be NULL when that size is 0. Calls that share a workspace must be
- * ordered on one stream.
+ * and, where the k range is split over several CTA pairs, which matrices of
+ * few rows are, the FP32 partial sums: splits x M x N floats; for Q5_K and
+ * Q4_0 the activations as FP16 terms). The size grows with M: one made for
+ * the longest prompt does for every shorter one, with the same results. A
+ * workspace that holds the activations but not the partial sums is taken,
+ * and K is not split. It may be NULL when the size is 0, and for Q5_K and
+ * Q4_0, which then run as passes of the decode GEMV. Calls that share a
+ * workspace must be ordered on one stream.
  * Replaces the tensor-core branch of linear_forward_batched_q4k_fp16 / _q6k_ /
  * _q8_0_ (quant.h:61,87,111; src/cuda/q4k_wmma.cu:56-332, q6k_wmma.cu:62-377,
  * q8_0_wmma.cu:54-309).

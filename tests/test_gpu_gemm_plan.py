@@ -7,7 +7,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 import oracle
-from brotensor_b200 import synth
+from brotensor_b200 import _capi, synth
 
 
 @pytest.mark.gpu
@@ -33,3 +33,27 @@ def test_long_prompts(fmt, N, K, M):
         ops.set_option("gemm_pair", 1)
     assert oracle.rel_l2(y.cpu().numpy(), one.cpu().numpy()) < 1e-5  # the order of the FP32 additions of a split K alone
     assert ops.device_status() == 0
+
+
+def _workspace(fmt, M, N, K, dtype=_capi.F16):
+    return _capi.lib().b200q_gemm_workspace_bytes(fmt, dtype, M, N, K)
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q5_K, synth.Q4_0])
+@pytest.mark.parametrize("N,K", [(4096, 4096), (1024, 4096), (14336, 4096), (4096, 14336), (640, 2560), (10240, 10240), (300, 1024), (257, 2048)])
+def test_a_workspace_covers_every_shorter_prompt(fmt, N, K):
+    sizes = [_workspace(fmt, M, N, K) for M in list(range(1, 1200)) + list(range(1200, 9000, 97))]
+    assert all(a <= b for a, b in zip(sizes, sizes[1:]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(4096, 4096), (1024, 4096)])
+def test_results_do_not_depend_on_a_larger_workspace(N, K):
+    from brotensor_b200 import ops
+    W = torch.from_numpy(synth.make_blocks(synth.Q4_K, N, K, seed=1)).cuda()
+    X = torch.from_numpy(synth.make_activations(2000, K, seed=2)).half().cuda()
+    ws = torch.empty(_workspace(synth.Q4_K, 2000, N, K), dtype=torch.uint8, device="cuda")
+    for M in (17, 45, 300, 512, 513, 1100, 2000):
+        own = torch.empty(_workspace(synth.Q4_K, M, N, K), dtype=torch.uint8, device="cuda")
+        a, b = (ops.gemm(synth.Q4_K, W, X[:M], N, out_dtype=torch.float32, ws=w) for w in (own, ws))
+        assert torch.equal(a, b), M
