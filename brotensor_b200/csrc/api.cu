@@ -63,6 +63,7 @@ int dp_get_tile_pairs();
 int dp_get_groups();
 int stream_get_option(int which);
 size_t gemm_tc_workspace_bytes(int fmt, int x_dtype, int M, int N, int K);
+int gemm_tc_check_ws(int fmt, const void* W, int x_dtype, int M, int N, int K, const void* ws, size_t ws_bytes);
 int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M,
                    int N, int K, void* ws, size_t ws_bytes, int sms, int* status, cudaStream_t st, bool* taken);
 
@@ -526,8 +527,13 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
     // (14336 x 4096: 46-48 us for any M up to 32), two passes of the small-batch GEMV on the integer tensor
     // cores take 28-30 us (Q4_K, Q8_0; 4096 x 4096: 14-15 against 18-20), and for Q6_K from 8192 rows two
     // passes of the warp-MMA GEMV 53-55 against 67. From 24 rows the GEMM is the faster one.
-    if (two_passes || (g_opt_gemm_path == 0 && M > 8 && M <= 16 && K <= 4096 &&
-        (((fmt == kQ4_K || fmt == kQ8_0) && (K == 2048 || K == 4096) && i8_get_enabled()) || (fmt == kQ6_K && N >= 8192)))) {
+    const bool old_passes = g_opt_gemm_path == 0 && M > 8 && M <= 16 && K <= 4096 &&
+                            (((fmt == kQ4_K || fmt == kQ8_0) && (K == 2048 || K == 4096) && i8_get_enabled()) || (fmt == kQ6_K && N >= 8192));
+    if (two_passes || old_passes) {
+        // (the calls that only gemv_hm has taken from the GEMM are held to the GEMM's workspace: which kernel is the faster one is no part of what a
+        // caller may leave out)
+        if (!old_passes)
+            if (int rc = gemm_tc_check_ws(fmt, W, x_dtype, M, N, K, ws, ws_bytes)) return rc;
         const size_t xs = (size_t)dt_size(x_dtype) * K, ys = (size_t)dt_size(y_dtype) * N;
         for (int m0 = 0; m0 < M; m0 += 8) {
             const int mm = M - m0 < 8 ? M - m0 : 8;

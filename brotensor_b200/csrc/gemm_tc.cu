@@ -306,6 +306,15 @@ static int launch_gemm_fmt(const GemmParams& p, size_t smem, cudaStream_t st) {
     return B200Q_OK;
 }
 
+// Whether a call of the tcgen05 GEMM's brings the workspace it needs.
+int gemm_tc_check_ws(int fmt, const void* W, int x_dtype, int M, int N, int K, const void* ws, size_t ws_bytes) {
+    if (!gemm_tc_takes(fmt, W, M, K)) return B200Q_OK;
+    const size_t need = gemm_tc_workspace_min_bytes(fmt, x_dtype, M, N, K);
+    if (!ws || ws_bytes < need) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
+    if (reinterpret_cast<uintptr_t>(ws) & 255) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace must be 256-byte aligned");
+    return B200Q_OK;
+}
+
 int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const void* bias, void* Y, int y_dtype, int M,
                    int N, int K, void* ws, size_t ws_bytes, int sms, int* status, cudaStream_t st, bool* taken) {
     (void)sms;
@@ -319,8 +328,7 @@ int launch_gemm_tc(int fmt, const void* W, const void* X, int x_dtype, const voi
     int split = ws && quads_ok ? gemm_split(fmt, M, N, K) : 1;
     if (split > 1 && ws_bytes < need + (size_t)split * M * N * sizeof(float)) split = 1;
     const GemmPlan plan = gemm_plan(fmt, M, N, K, split, split);
-    if (!ws || ws_bytes < need) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
-    if (reinterpret_cast<uintptr_t>(ws) & 255) return fail(B200Q_ERR_WORKSPACE, "gemm: workspace must be 256-byte aligned");
+    if (int rc = gemm_tc_check_ws(fmt, W, x_dtype, M, N, K, ws, ws_bytes)) return rc;
     const int tok_total = round_up16(M);
     {
         const long long total = (long long)(K / kBK) * tok_total * 8;

@@ -57,3 +57,21 @@ def test_results_do_not_depend_on_a_larger_workspace(N, K):
         own = torch.empty(_workspace(synth.Q4_K, M, N, K), dtype=torch.uint8, device="cuda")
         a, b = (ops.gemm(synth.Q4_K, W, X[:M], N, out_dtype=torch.float32, ws=w) for w in (own, ws))
         assert torch.equal(a, b), M
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt,N,K", [(synth.Q4_K, 2560, 2560), (synth.Q6_K, 1024, 4096), (synth.Q8_0, 640, 2560)])
+def test_nine_to_sixteen_rows_need_their_workspace(fmt, N, K):
+    """Also where the GEMM hands the call to two passes of the decode GEMV, which read none."""
+    from brotensor_b200 import ops
+    W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=1)).cuda()
+    room = torch.empty(_workspace(fmt, 16, N, K) + 256, dtype=torch.uint8, device="cuda")
+    for M in (9, 16):
+        X = torch.from_numpy(synth.make_activations(M, K, seed=2)).half().cuda()
+        y = torch.zeros(M, N, dtype=torch.float32, device="cuda")
+        for ws, n in ((None, 0), (room.data_ptr(), 1024), (room.data_ptr() + 16, room.numel() - 256)):
+            rc = _capi.lib().b200q_gemm(fmt, W.data_ptr(), X.data_ptr(), _capi.F16, None, y.data_ptr(), _capi.F32, M, N, K, ws, n, None)
+            assert rc == _capi.ERR_WORKSPACE
+        torch.cuda.synchronize()
+        assert not y.any()
+        assert ops.gemm(fmt, W, X, N, ws=room).any()
