@@ -48,6 +48,7 @@ static int static_scratch(void** out) {
 }
 
 size_t gemm_tc_workspace_min_bytes(int fmt, int x_dtype, int M, int N, int K);
+size_t gemm_mm_workspace_bytes(int fmt, int x_dtype, int M, int N, int K);
 
 }  // namespace b200q
 
@@ -67,11 +68,14 @@ int b200q_gemm_static(int fmt, const void* W, const void* X, int x_dtype, const 
                     "gemm_static: M %d x K %d needs %zu bytes of scratch, the built-in array holds %zu; "
                     "use b200q_gemm with a caller-owned workspace",
                     M, K, need, (size_t)kStaticScratchBytes);
+    // Q5_K and Q4_0 use the array where their prepared activations fit and run as passes of the decode GEMV where they do not.
+    const size_t mm = need == 0 && M > 8 ? gemm_mm_workspace_bytes(fmt, x_dtype, M, N, K) : 0;
+    const bool use = need > 0 || (mm > 0 && mm <= kStaticScratchBytes);
     void* scratch = nullptr;
-    if (need > 0)
+    if (use)
         if (int rc = static_scratch(&scratch)) return rc;
     // Same kernels, same routing and the same argument checks as the caller-workspace form.
-    return b200q_gemm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, scratch, need ? kStaticScratchBytes : 0, stream);
+    return b200q_gemm(fmt, W, X, x_dtype, bias, Y, y_dtype, M, N, K, scratch, use ? kStaticScratchBytes : 0, stream);
 }
 
 }  // extern "C"

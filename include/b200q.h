@@ -233,9 +233,12 @@ int b200q_gemm(int fmt, const void* W, const void* X, int x_dtype, const void* b
  * memory (b200q_gemm_static_max_bytes() bytes per device, 8 MiB: 512 tokens
  * at K = 8192, 1024 at K = 4096). For callers that cannot allocate: inside a
  * stream capture, under a fixed-footprint promise, or behind a plugin slot
- * that carries no workspace pointer. Problems whose
- * b200q_gemm_workspace_bytes() exceeds the array fail with
- * B200Q_ERR_WORKSPACE and nothing is launched.
+ * that carries no workspace pointer. Problems whose activation image exceeds
+ * the array fail with B200Q_ERR_WORKSPACE and nothing is launched; where the
+ * partial sums of a split K do not fit beside it, K is not split. Q5_K and
+ * Q4_0 run as b200q_gemm runs them where their prepared activations fit (4
+ * bytes per FP32 activation and 2 per 16-bit one, with a sixteenth more),
+ * and as passes of the decode GEMV above that.
  * All calls on one device share the one array: calls on the same stream are
  * ordered and safe; calls on different streams (or threads) that can overlap
  * race on it and must be ordered by the caller. Nothing in the array has to

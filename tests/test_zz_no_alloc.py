@@ -52,6 +52,25 @@ def test_static_matches_workspace_form_twice(fmt, N, K, M):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fmt", [synth.Q5_K, synth.Q4_0])
+def test_static_of_the_other_formats(fmt):
+    """Same kernel and bits as the workspace form while the prepared activations fit; passes of the decode GEMV, not an error, above."""
+    import ctypes
+    import torch
+    from brotensor_b200 import ops
+    last = ctypes.c_int(0)
+    for M, K, N, fits in ((20, 1024, 300, True), (400, 4096, 40, True), (1100, 4096, 40, False)):
+        W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=N + M)).cuda()
+        X = torch.from_numpy(synth.make_activations(M, K, seed=M)).cuda()
+        got = ops.gemm_static(fmt, W, X, N)
+        _capi.check(_capi.lib().b200q_get_option(b"last_kernel", ctypes.byref(last)))
+        ref = ops.gemm(fmt, W, X, N)
+        assert (last.value == 8) == fits and torch.equal(got, ref) == fits
+        assert torch.allclose(got, ref, rtol=1e-4, atol=1e-4 * float(ref.abs().max()))
+    assert ops.device_status() == 0
+
+
+@pytest.mark.gpu
 def test_static_small_m_routes_like_gemm():
     import torch
     from brotensor_b200 import ops
