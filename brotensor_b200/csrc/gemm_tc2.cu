@@ -40,7 +40,8 @@ struct PairParams {
     void* Y;
     int* status;
     int tokens, xp_tok_stride;
-    int tok_pass;        // blockIdx.z = z works on tokens [z * tok_pass, + tok_pass), at most 512 (a multiple of 16)
+    int tok_first;       // first token of this launch
+    int tok_pass;        // blockIdx.z = z works on tokens [tok_first + z * tok_pass, + tok_pass), at most 512 (a multiple of 16)
     int N, K, row_bytes;
     int bias_dtype, y_dtype;
     int n_a, n_b;        // ring depths in k-blocks: decoded weights (16 KB slots) and slabs; n_b <= n_a
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
     const uint32_t crank = cluster_ctarank();         // 0 = leader
     const int row0 = blockIdx.x * kGemmRows;          // the pair's CTAs own consecutive row tiles
     const int n_kb = p.n_split > 1 ? p.kb_split : p.K / kBK;  // k-blocks of this CTA; its first one is blockIdx.y * kb_split
-    const int t0 = (int)blockIdx.z * p.tok_pass, tokens = min(p.tok_pass, p.tokens - t0), tok_pad = (tokens + 15) & ~15;
+    const int t0 = p.tok_first + (int)blockIdx.z * p.tok_pass, tokens = min(p.tok_pass, p.tokens - t0), tok_pad = (tokens + 15) & ~15;
     const uint8_t* const xp = p.Xp + (size_t)t0 * 128u;
     const uint32_t tmem_cols = tok_pad <= 32 ? 32u : tok_pad <= 64 ? 64u : tok_pad <= 128 ? 128u : tok_pad <= 256 ? 256u : 512u;
     // token groups of up to 256: group g is one MMA of N = ng tokens into accumulator columns 256 g ..;
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_tc2_kernel(const PairPar
 // ---- host side ---------------------------------------------------------------------------------
 
 template <int FMT>
-static int launch_pair_fmt(const PairParams& p, size_t smem, cudaStream_t st) {
+static int launch_pair_fmt(const PairParams& p, int passes, size_t smem, cudaStream_t st) {
     auto kern = gemm_tc2_kernel<FMT>;
     static bool configured[64] = {};
     int dev = 0;
@@ -548,7 +549,7 @@ static int launch_pair_fmt(const PairParams& p, size_t smem, cudaStream_t st) {
     }
     const unsigned tiles = (unsigned)((p.N + kGemmRows - 1) / kGemmRows);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((tiles + 1u) & ~1u, (unsigned)(p.n_split > 1 ? p.n_split : 1), (unsigned)((p.tokens + p.tok_pass - 1) / p.tok_pass));  // whole pairs; a CTA past the last row tile decodes row N-1 and stores nothing
+    cfg.gridDim = dim3((tiles + 1u) & ~1u, (unsigned)(p.n_split > 1 ? p.n_split : 1), (unsigned)passes);  // whole pairs; a CTA past the last row tile decodes row N-1 and stores nothing
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -647,11 +648,16 @@ int launch_gemm_pair(int fmt, const void* W, const uint8_t* Xp, int tok_stride, 
     if (p.n_a > kPairMaxStages) p.n_a = kPairMaxStages;
     if (p.n_a < p.n_b) return fail(B200Q_ERR_UNSUPPORTED, "gemm: pair rings do not fit (%d weight slots, %d slab stages)", p.n_a, p.n_b);
     const size_t smem = (size_t)p.n_a * kb_a + (size_t)p.n_b * p.b_bytes + 1024;
-    int rc;
-    if (fmt == kQ4_K) rc = launch_pair_fmt<kQ4_K>(p, smem, st);
-    else if (fmt == kQ6_K) rc = launch_pair_fmt<kQ6_K>(p, smem, st);
-    else if (fmt == kQ6_KP) rc = launch_pair_fmt<kQ6_KP>(p, smem, st);
-    else rc = launch_pair_fmt<kQ8_0>(p, smem, st);
+    // (a grid has room for 65535 passes)
+    int rc = B200Q_OK;
+    for (long long t0 = 0; t0 < tokens && !rc; t0 += 65535LL * tok_pass) {
+        const int passes = (int)((tokens - t0 + tok_pass - 1) / tok_pass), now = passes < 65535 ? passes : 65535;
+        p.tok_first = (int)t0;
+        if (fmt == kQ4_K) rc = launch_pair_fmt<kQ4_K>(p, now, smem, st);
+        else if (fmt == kQ6_K) rc = launch_pair_fmt<kQ6_K>(p, now, smem, st);
+        else if (fmt == kQ6_KP) rc = launch_pair_fmt<kQ6_KP>(p, now, smem, st);
+        else rc = launch_pair_fmt<kQ8_0>(p, now, smem, st);
+    }
     if (rc || p.n_split == 1) return rc;
     const size_t quads = (size_t)tokens * N / 4;
     size_t blocks = (quads + 255) / 256;

@@ -75,3 +75,22 @@ def test_nine_to_sixteen_rows_need_their_workspace(fmt, N, K):
         torch.cuda.synchronize()
         assert not y.any()
         assert ops.gemm(fmt, W, X, N, ws=room).any()
+
+
+@pytest.mark.gpu
+def test_more_passes_than_a_grid_holds():
+    """One token into pass 65536 (activations and their image: 34 GB)."""
+    from brotensor_b200 import ops
+    fmt, M, N, K = synth.Q8_0, 65535 * 512 + 1, 4, 256
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("not enough free device memory")
+    W = torch.from_numpy(synth.make_blocks(fmt, N, K, seed=1)).cuda()
+    X = torch.zeros(M, K, dtype=torch.float16, device="cuda")
+    at = torch.tensor([0, 511, 512, M // 2, M - 514, M - 2, M - 1], device="cuda")
+    X[at] = torch.from_numpy(synth.make_activations(len(at), K, seed=2)).half().cuda()
+    y = ops.gemm(fmt, W, X, N, out_dtype=torch.float32)
+    want = ops.gemv(fmt, W, X[at].contiguous(), N, out_dtype=torch.float32)
+    assert oracle.rel_l2(y[at].cpu().numpy(), want.cpu().numpy()) < 2e-3
+    assert torch.count_nonzero(y) == len(at) * N
+    del X, y
+    torch.cuda.empty_cache()
