@@ -14,14 +14,20 @@ from .synth import BLOCK_BYTES, BLOCK_ELEMS
 _DT = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
 
 
+# The current device's index and a device's current stream as plain integers: torch's own short cuts where this torch has them (they are not
+# part of its public interface), else the public calls.
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _launch(t: torch.Tensor, f, *args) -> int:
     """f(*args, stream) with t's device current; the device is switched only when it is another one (entering and leaving
     torch.cuda.device and wrapping the stream in an object were a third of a small call's time on the host)."""
     i = t.device.index
-    if i == torch._C._cuda_getDevice():
-        return f(*args, torch._C._cuda_getCurrentRawStream(i))
+    if i is not None and i == _current_device():
+        return f(*args, _raw_stream(i))
     with torch.cuda.device(t.device):  # refuses a tensor that is not on a CUDA device
-        return f(*args, torch._C._cuda_getCurrentRawStream(i))
+        return f(*args, _raw_stream(i))
 
 
 def _check_w(fmt: int, W: torch.Tensor, N: int, K: int) -> None:

@@ -78,3 +78,39 @@ def test_compute_fails_loudly_without_a_gpu(L):
     rc = L.b200q_gemv(capi.Q4_K, p16, p16, capi.F32, None, p16, capi.F32, 1, 4, 256, None)
     assert rc == capi.ERR_CUDA
     assert b"CUDA error" in L.b200q_last_error()
+
+
+def _ops_without_torch_internals(monkeypatch):
+    import importlib.util
+    torch = pytest.importorskip("torch")
+    for name in ("_cuda_getDevice", "_cuda_getCurrentRawStream"):
+        monkeypatch.delattr(torch._C, name, raising=False)
+    spec = importlib.util.spec_from_file_location("brotensor_b200._ops_public", os.path.join(ROOT, "brotensor_b200", "ops.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod, torch
+
+
+def test_ops_loads_on_a_torch_without_the_short_cuts(monkeypatch):
+    mod, torch = _ops_without_torch_internals(monkeypatch)
+    assert mod._current_device is torch.cuda.current_device
+    with pytest.raises(ValueError):  # a host tensor is refused before any CUDA call
+        mod._launch(torch.zeros(1), lambda *a: 0)
+
+
+@pytest.mark.gpu
+def test_ops_runs_on_a_torch_without_the_short_cuts(monkeypatch):
+    from brotensor_b200 import ops, synth
+    import torch
+    W = torch.from_numpy(synth.make_blocks(synth.Q4_K, 64, 512, seed=1)).cuda()
+    x = torch.from_numpy(synth.make_activations(1, 512, seed=2)).cuda()
+    want = ops.gemv(synth.Q4_K, W, x, 64)
+    with monkeypatch.context() as m:  # (the public calls need the internals again)
+        mod, _ = _ops_without_torch_internals(m)
+    assert mod._raw_stream is not ops._raw_stream
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        y = mod.gemv(synth.Q4_K, W, x, 64)
+    side.synchronize()
+    assert torch.equal(y, want)
