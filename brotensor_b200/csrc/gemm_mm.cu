@@ -151,16 +151,6 @@ __global__ void __launch_bounds__(256) gemm_mm_prep_kernel(const void* X, int x_
 }
 
 // ---- the GEMM -------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_f16_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void mma_f16_add(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
@@ -288,16 +278,16 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
                         if constexpr (SPLIT) ldsm4(baddr + (uint32_t)(p.off_lo - p.off_b) + (uint32_t)(n0 + n) * 4096u, y[n]);
                     }
 #pragma unroll
-                    for (int n = 0; n < GN; ++n) mma_f16_zero(c[n], a[0], b[0], a[1], b[1], x[n][0], x[n][1]);
+                    for (int n = 0; n < GN; ++n) qm_mma_zero<false>(c[n], a[0], b[0], a[1], b[1], x[n][0], x[n][1]);
                     if constexpr (SPLIT) {
 #pragma unroll
-                        for (int n = 0; n < GN; ++n) mma_f16_add(c[n], a[0], b[0], a[1], b[1], y[n][0], y[n][1]);
+                        for (int n = 0; n < GN; ++n) qm_mma<false>(c[n], a[0], b[0], a[1], b[1], y[n][0], y[n][1]);
                     }
 #pragma unroll
-                    for (int n = 0; n < GN; ++n) mma_f16_add(c[n], a[2], b[2], a[3], b[3], x[n][2], x[n][3]);
+                    for (int n = 0; n < GN; ++n) qm_mma<false>(c[n], a[2], b[2], a[3], b[3], x[n][2], x[n][3]);
                     if constexpr (SPLIT) {
 #pragma unroll
-                        for (int n = 0; n < GN; ++n) mma_f16_add(c[n], a[2], b[2], a[3], b[3], y[n][2], y[n][3]);
+                        for (int n = 0; n < GN; ++n) qm_mma<false>(c[n], a[2], b[2], a[3], b[3], y[n][2], y[n][3]);
                     }
 #pragma unroll
                     for (int n = 0; n < GN; ++n) {
@@ -320,7 +310,7 @@ __global__ void __launch_bounds__(kMmMaxWarps * 32, 1) gemm_mm_kernel(const __gr
                     for (int n = 0; n < NT; ++n) {
                         const uint2 x = ls64(smem + slot * p.stage_bytes + p.off_s + (8 * n + g) * 32 + 8 * t);
                         float c[4];
-                        mma_f16_zero(c, m0, m1, m0, m1, x.x, x.y);
+                        qm_mma_zero<false>(c, m0, m1, m0, m1, x.x, x.y);
                         acc[n][0] = fmaf(fA, c[0], acc[n][0]);
                         acc[n][1] = fmaf(fA, c[1], acc[n][1]);
                         acc[n][2] = fmaf(fB, c[2], acc[n][2]);

@@ -46,28 +46,6 @@ struct HmParams {
     int row_q, row_r;  // CTA b owns row_q + (b < row_r) rows
 };
 
-template <bool BF>
-__device__ __forceinline__ void hm_mma_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    if constexpr (BF)
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-            : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-    else
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-            : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-template <bool BF>
-__device__ __forceinline__ void hm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    if constexpr (BF)
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
@@ -290,22 +268,22 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
                 hm_quants<FMT, BF>(rb, s, t, b);
                 hm_scales<FMT, BF>(ra, dA, sc[0][0], sc[0][1], s, fA);
                 hm_scales<FMT, BF>(rb, dB, sc[1][0], sc[1][1], s, fB);
-                hm_mma_zero<BF>(c, a[0], b[0], a[1], b[1], x[0], x[1]);
+                qm_mma_zero<BF>(c, a[0], b[0], a[1], b[1], x[0], x[1]);
                 if constexpr (FMT == kQ6_K) {
                     float c2[4];
-                    hm_mma_zero<BF>(c2, a[2], b[2], a[3], b[3], x[2], x[3]);
+                    qm_mma_zero<BF>(c2, a[2], b[2], a[3], b[3], x[2], x[3]);
                     acc[0] = fmaf(fA[1], c2[0], acc[0]);
                     acc[1] = fmaf(fA[1], c2[1], acc[1]);
                     acc[2] = fmaf(fB[1], c2[2], acc[2]);
                     acc[3] = fmaf(fB[1], c2[3], acc[3]);
                 } else {
-                    hm_mma<BF>(c, a[2], b[2], a[3], b[3], x[2], x[3]);
+                    qm_mma<BF>(c, a[2], b[2], a[3], b[3], x[2], x[3]);
                 }
                 if constexpr (FMT == kQ8_0 && BF) {
                     hm_quants<FMT, BF, true>(ra, s, t, a);
                     hm_quants<FMT, BF, true>(rb, s, t, b);
-                    hm_mma<BF>(c, a[0], b[0], a[1], b[1], x[0], x[1]);
-                    hm_mma<BF>(c, a[2], b[2], a[3], b[3], x[2], x[3]);
+                    qm_mma<BF>(c, a[0], b[0], a[1], b[1], x[0], x[1]);
+                    qm_mma<BF>(c, a[2], b[2], a[3], b[3], x[2], x[3]);
                 }
                 acc[0] = fmaf(fA[0], c[0], acc[0]);
                 acc[1] = fmaf(fA[0], c[1], acc[1]);
@@ -315,8 +293,8 @@ __global__ void __launch_bounds__(kHmMaxWarps * 32, 1) gemv_hm_kernel(const __gr
                     const uint32_t sel = 0x4040u | (uint32_t)((s & 3) * 0x101);
                     const uint32_t m0 = hm_halves<BF>(s < 4 ? mn[0][0] : mn[0][1], sel, 0);
                     const uint32_t m1 = hm_halves<BF>(s < 4 ? mn[1][0] : mn[1][1], sel, 0);
-                    hm_mma<BF>(cm, m0, m1, m0, m1, x[0], x[1]);
-                    hm_mma<BF>(cm, m0, m1, m0, m1, x[2], x[3]);
+                    qm_mma<BF>(cm, m0, m1, m0, m1, x[0], x[1]);
+                    qm_mma<BF>(cm, m0, m1, m0, m1, x[2], x[3]);
                 }
             }
             if constexpr (F::mins) {

@@ -95,6 +95,30 @@ __device__ __forceinline__ uint32_t k_scales_hi(const uint4& h) { return (h.w & 
 __device__ __forceinline__ uint32_t k_mins_lo(const uint4& h) { return h.z & 0x3f3f3f3fu; }
 __device__ __forceinline__ uint32_t k_mins_hi(const uint4& h) { return ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u); }
 
+// D = A * B (+ D), 16 x 8 x 16, FP16 or BF16 operands and FP32 sums.
+template <bool BF>
+__device__ __forceinline__ void qm_mma_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+template <bool BF>
+__device__ __forceinline__ void qm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // Eight activations of row m from element k on: raw (the second word for FP32 only), and as floats.
 __device__ __forceinline__ void qm_load_raw(const void* X, bool f32, int K, int m, int k, uint4 (&r)[2]) {
     const uint8_t* x = static_cast<const uint8_t*>(X) + ((size_t)m * K + k) * (f32 ? 4 : 2);
