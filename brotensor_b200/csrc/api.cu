@@ -292,24 +292,29 @@ static int gemv_streaming(DevInfo* d, int fmt, const void* W, const void* X, int
 }
 
 // Which decode calls go to the two raw-quant MMA kernels (gemv_hm.cu: 16-bit activations; gemv_mb.cu: any). Both do a call of
-// few weight rows per SM in little more than a launch, whatever M is, and stream long matrices at half the memory's
-// rate, so the lines lie where the older kernels' times cross theirs (us, old -> gemv_hm, FP16, overlapped launches):
-//   Q4_K   M = 2: 1024 x 4096 4.6 -> 3.7, 6912 x 2560 7.7 -> 6.3, 4096 x 14336 15.9 -> 17.9, 14336 x 4096 12.5 -> 19.1
-//          M = 6: 4096 x 4096 10.6 -> 6.5, 4096 x 14336 49 -> 18.5, 2560 x 6912 22 -> 9.6, 14336 x 4096 (integer MMA) 18.1 -> 19.0
-//   Q6_K   M = 2: 1024 x 4096 5.0 -> 4.5, 2048 x 4096 5.9 -> 5.5, 1024 x 8192 7.2 -> 7.2, 2048 x 8192 8.3 -> 8.8, 2048 x 14336 12.7 -> 14.3,
-//          4096 x 4096 7.7 -> 8.3; M = 3: 2048 x 14336 16.9 -> 14.7; M = 6: 10.3 -> 8.7, 4096 x 14336 43 -> 25, 14336 x 4096 22 -> 25
-//   Q8_0   M = 2: 4096 x 4096 10.9 -> 7.7, 4096 x 14336 19.8 -> 21.6; M = 6: 11.4 -> 7.9, 43.6 -> 22, 14336 x 4096 18.8 -> 21.9
-// Rows of Q6_K that are not whole runs of eight blocks, Q5_K and Q4_0 had the plain-load kernel (2560 x 6912, M = 1: 20.8 -> 11.6,
-// 24.8 -> 10.2, 19.8 -> 8.0); from M = 1, 2 and many rows gemv_mb is the faster of the two for the 4- and 5-bit formats (14336 x 4096
-// Q5_K 21.6 against 17.1, 32003 x 2560 Q6_K 33.3 against 27.3, 32000 x 4096 Q4_0 32.8 against 30.8).
+// few weight rows per SM in little more than a launch, whatever M is, and stream long matrices at a quarter to a half of the memory's
+// rate, so the lines lie where the older kernels' times cross theirs (us, old -> gemv_hm, FP16, one box):
+//   Q4_K   M = 2: 1024 x 4096 4.5 -> 3.9, 2048 x 4096 5.2 -> 4.6, 3072 x 4096 5.8 -> 6.3, 4096 x 4096 6.3 -> 6.6, 6912 x 2560 7.8 -> 6.5,
+//          8192 x 2048 7.6 -> 6.5, 2560 x 6912 7.8 -> 9.2, 4096 x 14336 15.2 -> 17.4
+//          M = 6: 4096 x 4096 10.8 -> 6.7, 4096 x 14336 48.6 -> 19.2, 2560 x 6912 22.4 -> 9.9, 32003 x 2560 28.9 -> 23.0; on the integer MMA
+//          (K = 2048, 4096) 14336 x 4096 18.8 -> 18.1, 32000 x 4096 28.2 -> 32.7
+//   Q6_K   M = 2: 1024 x 4096 5.1 -> 4.5, 2048 x 4096 5.9 -> 5.5, 1024 x 8192 7.2 -> 7.2, 2048 x 8192 8.3 -> 8.8, 2048 x 14336 12.7 -> 14.3,
+//          4096 x 4096 7.9 -> 8.4; M = 3: 2048 x 14336 16.9 -> 14.7; M = 6: 4096 x 4096 10.5 -> 8.9, 4096 x 14336 44.3 -> 25.7,
+//          14336 x 4096 23.0 -> 23.8, 32000 x 4096 43.4 -> 43.7
+//   Q8_0   M = 2: 4096 x 4096 11.4 -> 8.0, 8192 x 4096 15.2 -> 13.3, 4096 x 14336 20.7 -> 21.4; M = 6: 4096 x 4096 11.7 -> 8.2, 4096 x 14336 43.8 -> 23.2,
+//          14336 x 4096 19.7 -> 20.3; M = 8: 32000 x 8192 81.5 -> 87.1 (but M = 3: 32003 x 2560 34.4 -> 26.5, beyond the line)
+// Rows of Q6_K that are not whole runs of eight blocks, Q5_K and Q4_0 have gemv_mb on the other side (before either: the plain-load kernel, one
+// row of 2560 x 6912 20.8, 24.8 and 19.8 us): Q4_0 is gemv_hm's altogether (one row, 14336 x 4096 18.6 -> 16.4, 32000 x 4096 32.9 -> 29.7,
+// 24576 x 2560 18.2 -> 17.3), one and two rows of the others while they are few (one row, Q5_K 4096 x 4096 7.6 -> 7.1, 8192 x 4096 12.0 -> 12.3,
+// 14336 x 4096 18.1 -> 20.8; Q6_K 2560 x 6912 12.6 -> 12.0, 32003 x 2560 29.9 -> 31.2).
 static bool hm_wanted(int fmt, int x_dtype, int M, int N, int K) {
     if (x_dtype == B200Q_DT_F32) return false;
     if (hm_get_enabled() == 2) return true;
     const bool few = N <= 8192;
     switch (fmt) {
         case kQ5_K: return M > 2 || few;
-        case kQ4_0: return M > 2 || N <= 16384;
-        case kQ4_K: return M == 2 ? K <= 4096 && (long long)N * K <= 18000000 : M > 2 && (few || (M >= 4 && K != 2048 && K != 4096));
+        case kQ4_0: return true;
+        case kQ4_K: return M == 2 ? K <= 4096 && (long long)N * K <= (K > 2560 ? 2048 * 4096 : 18000000) : M > 2 && (few || (M >= 4 && K != 2048 && K != 4096));
         case kQ6_K: return K % kQ6RunElems != 0 ? M > 2 || few : M >= 4 ? few : M >= 2 && N <= 2048 && (M > 2 || (long long)N * K <= 2048 * 4096);
         case kQ8_0: return M >= 2 && (few ? M > 2 || K <= 8192 : M > 2 && K != 2048 && K != 4096 && N <= 16384);
     }

@@ -99,13 +99,14 @@ def test_matrices_of_few_rows_and_many_activations(fmt, N, K, ops_raw):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,K,M,kernel", [(2048, 4096, 2, HM), (2048, 8192, 2, DP), (1024, 14336, 2, DP), (2048, 14336, 3, HM)])
-def test_two_rows_of_q6k(N, K, M, kernel, ops_raw):
-    """Two rows of a longer Q6_K matrix are the integer-dot kernel's."""
-    W, x, b, want = _operands(synth.Q6_K, N, K, M, "f16")
-    y = ops_raw.gemv(synth.Q6_K, W, x, N, bias=b, out_dtype=torch.float32)
+@pytest.mark.parametrize("fmt,N,K,M,kernel", [(synth.Q6_K, 2048, 4096, 2, HM), (synth.Q6_K, 2048, 8192, 2, DP), (synth.Q6_K, 1024, 14336, 2, DP),
+                                              (synth.Q6_K, 2048, 14336, 3, HM), (synth.Q4_K, 2048, 4096, 2, HM), (synth.Q4_K, 3072, 4096, 2, DP),
+                                              (synth.Q4_K, 6912, 2560, 2, HM), (synth.Q4_0, 20000, 512, 1, HM), (synth.Q5_K, 9000, 512, 1, MB)])
+def test_where_the_lines_lie(fmt, N, K, M, kernel, ops_raw):
+    W, x, b, want = _operands(fmt, N, K, M, "f16")
+    y = ops_raw.gemv(fmt, W, x, N, bias=b, out_dtype=torch.float32)
     assert _last_kernel() == kernel
-    assert oracle.rel_l2(y.cpu().numpy(), want) < (2e-6 if kernel == HM else 2e-3)  # (15-bit fixed point in the other)
+    assert oracle.rel_l2(y.cpu().numpy(), want) < (2e-3 if kernel == DP else 2e-6)  # (15-bit fixed point in the integer-dot kernel)
 
 
 @pytest.mark.gpu
