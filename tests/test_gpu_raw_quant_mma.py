@@ -1,6 +1,8 @@
 """The kernels that multiply raw quants on the warp-level tensor-core instructions - csrc/gemv_hm.cu (16-bit activations, 1..8 rows), csrc/gemv_mb.cu
-(Q5_K, Q4_0, Q6_K with any activations, 1..8 rows) and csrc/gemm_mm.cu (Q5_K, Q4_0, from nine tokens) - against the oracle's 64-bit sums. Nothing in them is rounded below
-FP32: exact products, sums of a few hundred FP32 terms (at most sqrt(K / 32 + 16) * 2^-24 < 2e-6 over a row for K <= 14336), so that is the bound.
+(Q5_K, Q4_0, Q6_K with any activations, 1..8 rows) and csrc/gemm_mm.cu (Q5_K, Q4_0, from nine tokens) - against the oracle's 64-bit sums.
+gemv_hm multiplies the activations as they are; the other two hold them in fixed point (30 bits, 62 for one FP32 row) or as FP16 terms (22 bits of
+each value) and leave rows that these do not hold to a plain FP32 loop, so in all of them a result is a sum of a few hundred FP32 terms with
+errors of at most 2^-22 each (sqrt(K / 32 + 16) * 2^-24 and less than 2^-21 for the terms: below 2e-6 over a row for K <= 14336), which is the bound.
 Sizes: one row, ragged tiles of 16, fewer rows than SMs, several row tiles per CTA, several passes over a CTA's rows, K of one block, of
 an odd number of blocks (Q6_K rows that start on any even byte) and of more blocks than a CTA has warps."""
 import ctypes
@@ -13,7 +15,7 @@ torch = pytest.importorskip("torch")
 import oracle
 from brotensor_b200 import _capi, synth
 
-DP, HM, MB, MM = 3, 6, 7, 8  # what the option "last_kernel" calls them
+PLAIN, DP, HM, MB, MM = 1, 3, 6, 7, 8  # what the option "last_kernel" calls them
 FMTS = [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0, synth.Q4_0]
 SHAPES = [(1, 256), (15, 512), (37, 768), (300, 6912), (2373, 1024), (40, 14336), (20000, 256)]
 DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
@@ -78,7 +80,9 @@ def test_a_few_dozen_tokens(fmt, N, K, ops_raw):
         if N * K * M > 4e8:
             continue
         W, x, b, want = _operands(fmt, N, K, M, dtype)
+        ops.set_option("gemv_hm", 0)  # (up to sixteen rows of 16-bit activations are its)
         y = ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32)
+        assert _last_kernel() == MM, (M, dtype)
         assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (M, dtype)
         assert torch.equal(y, ops.linear(fmt, W, x, N, bias=b, out_dtype=torch.float32))
 
@@ -121,7 +125,8 @@ def test_weights_on_two_byte_boundaries(ops_raw):
             moved = buf[shift:shift + W.numel()]
             moved.copy_(W.reshape(-1))
             y = ops.linear(fmt, moved, x, N, bias=b, out_dtype=torch.float32)
-            assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-3
+            assert _last_kernel() == (PLAIN if fmt != synth.Q6_K else MB if dtype == "f32" else HM), (fmt, shift, M)
+            assert oracle.rel_l2(y.cpu().numpy(), want) < 2e-6, (fmt, shift, M)
 
 
 @pytest.mark.gpu
