@@ -19,7 +19,7 @@
 // each 256-k stage by sub-blocks and add up at the end in a fixed order). Stages of 256 k - raw rows and activations - are fetched with
 // cp.async two or three ahead, one CTA barrier per stage. What bounds it at 48 tokens: the latency of its instructions with three to
 // four warps per scheduler (about 1.9 times the cycles that its MMAs and its reads of B take).
-// 96 tokens, 14336 x 4096: Q5_K 103 us, Q4_0 80 (twelve passes of the plain-load GEMV before: 0.85 ms, 0.7 ms); 16 tokens 36 and 26
+// 96 FP16 tokens, 14336 x 4096: Q5_K 106 us, Q4_0 82 (twelve passes of the plain-load GEMV before: 0.85 ms, 0.7 ms); 16 tokens 37 and 28
 // (147, 126).
 //
 // Takes the place of what brotensor's fused-dequant WMMA kernels are for its formats (src/cuda/q4k_wmma.cu:56-310).

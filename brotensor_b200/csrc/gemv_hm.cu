@@ -1,5 +1,5 @@
 // Decode GEMV on warp-level FP16 / BF16 MMA for activations of these types, 1..8 rows, every block format, K a multiple of 256 (sm_100a):
-// Y(M, N) = X(M, K) * decode(W(N, K))^T with FP32-class accuracy, at the speed of the weight stream.
+// Y(M, N) = X(M, K) * decode(W(N, K))^T with FP32-class accuracy, at nearly the same time for any M.
 //
 // The activations are multiplied as they lie in memory: an FP16 or BF16 value is an MMA operand, so there is no staging pass, no scale and
 // no rounding. The weights' quants become integers of the same type in a mask, a byte permute and a packed subtraction per two (their offsets -
@@ -8,15 +8,15 @@
 // Each sub-block's products are summed on the tensor cores in FP32 and multiplied by its scale in FP32 (four FMA per 16 x 8 x 32
 // products). The minimums of Q4_K / Q5_K go through the same B fragments: an MMA whose A operand is the sub-block's 6-bit min in
 // every lane accumulates sum(m * x) over a block, one FMA with dmin per block.
-// A k-step of 16 rows x 32 k is two (with mins four) MMAs and some seventy instructions whatever M is, more than half of them on the
-// half-rate integer pipe: 37 of the SM's cycles against the 12 that its bytes take from memory (IPC 1.8; the largest stall is
-// the barrier between stages, no pipe is above 35 %). So a call of few rows per SM costs little more than a launch, and a long
-// matrix streams at a third of the memory's rate; 20 and 24 warps instead of 14 are no faster.
+// A k-step of 16 rows x 32 k is two (with mins four) MMAs and some eighty instructions whatever M is, half of them on the half-rate integer
+// pipe, against the 12 cycles that its bytes take from memory. Six rows of 14336 x 4096 Q4_K: 18.1 us, 28 % of the memory's rate, IPC 2.05, no pipe
+// above 40 %; 32000 x 4096 32.7 us, 35 %. So a call of few rows per SM costs little more than a launch, and long matrices stay with the
+// kernels that have fewer instructions per weight where there are any; 20 and 24 warps instead of 14 are no faster.
 //
 // A CTA owns an even share of the rows, up to eight 16-row tiles at a time, and its warps are tiles x blocks: a stage holds as many
 // neighbouring 256-element blocks of the rows (and of X) as there are warps per tile, each warp multiplies one of them, and the tile's
 // warps add up at the end of the rows in a fixed order. So every warp has eight k-steps of independent work between two CTA
-// barriers however few rows there are (with stages of one block, shared by sub-blocks, 4096 x 14336 took 33 us instead of 17.6). Stages
+// barriers (the staged form's largest stall) however few rows there are (with stages of one block, shared by sub-blocks, 4096 x 14336 took 33 us instead of 17.6). Stages
 // are fetched with cp.async up to five ahead. Where the rows take many steps and the activations are short they are kept in shared memory
 // whole, every warp has a ring of its own and no barrier is left in the loop.
 // Results that are not finite are computed again in plain FP32 (qm_plain_rows): 0 * inf on a masked quant is not what the

@@ -25,9 +25,10 @@
 //     warp of the current tile. The order of the additions is fixed (reproducible results).
 //   * The minimums' term of Q5_K, sum over sub-blocks of dmin * m * sum(x), is one TF32 MMA per column set: the
 //     6-bit mins are exact in TF32 and the FP32 sums of x are split over the planes' columns in pieces of 11 bits.
-// Measured (one row, us, plain-load kernel -> this one): Q5_K 14336 x 4096 39.8 -> 17.1, 4096 x 4096 16.9 -> 7.4, 4096 x 14336 50.6 -> 19.5; Q4_0 29.5 -> 17.6,
-// 13.1 -> 7.1, 40.4 -> 19.4; Q6_K 2560 x 6912 20.8 -> 12.4. It runs at half of the memory's rate for one row: 58 instructions per k-step of
-// 16 x 32, of which the kernel's own work is about 25 and the rest is waiting for the others at a tile's end.
+// Measured (one FP32 row, us, plain-load kernel -> this one): Q5_K 14336 x 4096 39.8 -> 18.3, 4096 x 4096 16.9 -> 8.3, 4096 x 14336 50.6 -> 21.9; Q4_0 29.5 -> 19.0,
+// 13.1 -> 7.6, 40.4 -> 21.4; Q6_K 2560 x 6912 20.8 -> 13.2. 14336 x 4096 is 2.2 TB/s of Q5_K and 1.7 of Q4_0, 34 and 27 % of the memory's rate: 58
+// instructions per k-step of 16 x 32, of which the kernel's own work is about 25 and the rest is waiting for the others at a tile's end.
+// Three and more rows spill (128 registers, 60 .. 840 bytes): staging, not the loop.
 // Rows of activations that are not finite or not held, and all rows where a result is not finite, take a plain FP32 loop at the end of the
 // launch (qm_plain_rows): an integer sum of zero times an infinite scale is not what the decoded weights give.
 //

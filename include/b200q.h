@@ -42,8 +42,8 @@ extern "C" {
 #define B200Q_FMT_Q6_K 24 /* 256 elements / 210 B: u8 ql[128], u8 qh[64], i8 scales[16], fp16 d */
 /*
  * Two more GGUF formats that brotensor's loader carries as opaque storage with no op behind them
- * (src/gguf.cpp:111-130); layouts as ggml defines them. Decode, dequant, decode GEMV, GEMM (as passes
- * of the GEMV) and the row gather take them; the tensor-core prefill kernel and the sharded head do not.
+ * (src/gguf.cpp:111-130); layouts as ggml defines them. Decode, dequant, decode GEMV, GEMM (warp-level tensor
+ * cores) and the row gather take them; the tcgen05 prefill kernel, the fused forms and the sharded head do not.
  */
 #define B200Q_FMT_Q4_0 10 /*  32 elements /  18 B: fp16 d, u8 qs[16]; w = d * (nibble - 8), element j < 16 the low nibble of qs[j], else the high nibble of qs[j - 16] */
 #define B200Q_FMT_Q5_K 23 /* 256 elements / 176 B: fp16 d, fp16 dmin, u8 scales[12] (packed as in Q4_K), u8 qh[32], u8 qs[128]; w = d * sc * (nibble + 16 * bit) - dmin * m */
@@ -290,8 +290,8 @@ int b200q_device_status(int* status_out);
  *                 one pipeline with 32-row tiles; "gemv_split_full" (Q6_K only) -1 = automatic, 0 = one full
  *                 barrier per stage, 1 = one per consumer warp and stage
  *   "gemm_path"   0 = automatic (tcgen05 GEMM from 9 rows, except 9..16 rows of Q4_K / Q8_0 with K = 2048 / 4096 and
- *                 of Q6_K from 8192 weight rows, and of matrices up to 8192 rows with 16-bit activations, which run as
- *                 two passes of the small-batch GEMV; Q5_K and Q4_0: "gemm_mm"), 1 = passes of the
+ *                 of Q6_K from 8192 weight rows with K <= 4096, and of raw-layout matrices up to 8192 rows with 16-bit
+ *                 activations, which run as two passes of the small-batch GEMV; Q5_K and Q4_0: "gemm_mm"), 1 = passes of the
  *                 decode GEMV only, 2 = the tcgen05 GEMM or an error
  *   "gemm_pair"   0 = one-CTA tcgen05 kernel, otherwise the CTA-pair kernel (default)
  *   "gemm_split"  0 = never split K; 1 (default) = where it shortens the call, matrices of few row tiles
@@ -300,7 +300,7 @@ int b200q_device_status(int* status_out);
  *   "gemv_xr"     Q4_K / Q6_K, one activation row, K <= 4096: 1 = the activation-resident kernel where it is the
  *                 faster one (default), 2 = for every such call, 0 = never
  *   "gemv_hm"     FP16 / BF16 activations, 1..8 rows: 1 = the raw-quant tensor-core kernel where it is the faster one (default),
- *                 2 = for every such call, 0 = never
+ *                 2 = for every such call (K a multiple of 256, raw blocks, weights on 16 bytes; Q6_K anywhere), 0 = never
  *   "gemv_mb"     Q5_K, Q4_0, Q6_K, 1..8 rows: 1 = the integer tensor-core kernel for calls that would else go to the plain-load
  *                 kernel (default), 2 = for every such call "gemv_hm" leaves, 0 = never
  *   "gemm_mm"     Q5_K, Q4_0 from 9 rows: 1 = the warp-level tensor-core GEMM (default), 0 = passes of the decode GEMV

@@ -33,8 +33,9 @@ void linear_forward_batched_q6k_fp16(const Tensor& W_q6k, const Tensor* bias, co
 
 // Extension: Q4_0 and Q5_K, which brotensor's GGUF loader hands out as opaque storage with no op behind
 // them (src/gguf.cpp:111-130). Same three ops, shapes, dtypes and errors as for the formats above; the
-// decode follows ggml's block definitions. They run on the plain-load GEMV (weights read once for up to
-// eight activation rows), not on the streaming and tensor-core kernels.
+// decode follows ggml's block definitions. They run on warp-level tensor-core kernels that read the raw quants
+// (up to eight activation rows read the weights once; more rows in passes of up to 64 tokens), and on the plain-load GEMV
+// where K is no multiple of 256 or the weights are not on a 16-byte boundary; there is no tcgen05, fused or sharded form.
 void dequant_q4_0_to_fp16(const Tensor& W_q4_0, Tensor& W_fp16);
 void linear_forward_q4_0_fp16(const Tensor& W_q4_0, const Tensor* bias, const Tensor& x, Tensor& y);
 void linear_forward_batched_q4_0_fp16(const Tensor& W_q4_0, const Tensor* bias, const Tensor& X_BD, Tensor& Y_BD);
